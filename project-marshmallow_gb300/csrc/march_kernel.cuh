@@ -556,6 +556,20 @@ struct Ray {
     bool killed;    // rd.y < 0: stored as is (:351-354)
 };
 
+// March distance at which a ray from the camera is past relative height 0.9 for good.  The cloud
+// layer's profiles (layer_fast) end there, so every later cloudTest of the ray is 0: nothing is
+// accumulated, and the ray's colour and depth are what they are.  The ray rises (rays below the horizon
+// are not marched) and the earth centre lies straight below the camera, so |pos - centre| grows with
+// t; p.end_h is the camera's height over the centre and p.end_c = r^2 - end_h^2 for r = the radius at
+// relative height 0.9 plus 40 m, far more than the float error of a sample's height (march_host_consts;
+// +INF where it does not hold or where the caller counts the shader's samples).  The samples left out
+// are 3.2% of the cloudTest calls of a sweep frame; the texture unit bounds a frame, so it gains what
+// they cost: 3840x2160 2983 -> 2913 us, 1920x1080 857 -> 838 us (pitch 15, sun 30), same bits.
+__device__ __forceinline__ float shell_end(const MarchLaunch& p, float rdy) {
+    const float b = p.end_h * rdy;
+    return sqrtf(b * b + p.end_c) - b;
+}
+
 template <bool E, int S>
 __device__ __forceinline__ Ray ray_setup(const MarchLaunch& p, const Frame& f, int px, int py) {
     const mm_uniforms& u = p.u;
@@ -627,6 +641,9 @@ __device__ __forceinline__ Ray ray_setup(const MarchLaunch& p, const Frame& f, i
         r.bg = bg + sunDisk;
         r.alpha = sunDisk;
     }
+    // Production arithmetic: past relative height 0.9 the layer profile is zero whatever the weather
+    // map holds, so no later sample changes the ray (shell_end).
+    if (!E) r.t1 = fminf(r.t1, shell_end(p, rd.y));
     r.cosTheta = dot(rd, f.sunDir);  // :386
     r.hg = fmaxf(hgPhase<E>(r.cosTheta, 0.6f), 0.7f * hgPhase<E>(r.cosTheta, 0.99f - 0.1f));  // :407
     return r;

@@ -95,6 +95,7 @@ struct MarchLaunch {
     // (march_host_consts) so the kernels read them from the parameter bank instead of holding them
     // in registers: the normalized sun direction and 20 * wind.
     float sun_dir[3], wind20[3];
+    float end_h, end_c;  // where a ray leaves the cloud layer for good (march_kernel.cuh, shell_end)
     float cone[18];  // the six sun-cone offsets mat3(directionBasis) * v (compute-clouds.comp:392-401)
 };
 
@@ -144,6 +145,14 @@ inline void march_host_consts(MarchLaunch& p) {
         p.sun_dir[i] = b[i] * inv;
         p.wind20[i] = 20.0f * p.u.sky.wind[i];
     }
+    // Camera height over the earth centre and (radius at relative height 0.9 + 40 m)^2 - height^2.  The
+    // bound on a sample's height error holds for cameras within 1000 km of the origin; a launch that
+    // counts the shader's samples runs them all.
+    const float* c = p.u.camera.camera_position;
+    const double h = (double)c[1] + 995000.0, re = 1.0e6 + 0.9 * 20000.0 + 40.0;
+    const bool ends = !p.counters && fabsf(c[0]) <= 1.0e6f && fabsf(c[1]) <= 9.0e5f && fabsf(c[2]) <= 1.0e6f;
+    p.end_h = (float)h;
+    p.end_c = ends && h < re ? (float)(re * re - h * h) : INFINITY;
     static const float v[6][3] = {{0.0f, 0.6f, 0.0f}, {0.0f, 0.5f, 0.05f}, {0.1f, 0.75f, 0.0f},
                                   {0.2f, 2.5f, 0.3f}, {0.0f, 6.0f, 0.0f},  {-0.1f, 1.0f, -0.2f}};
     const float* m = p.u.sun.direction_basis;
