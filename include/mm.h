@@ -277,9 +277,9 @@ typedef enum mm_math_mode {
 typedef enum mm_schedule {
     MM_SCHEDULE_TILED = 0,      /* one thread marches one pixel start to end (the shader's own loop
                                    nest), 8x4 pixel tiles per warp, block rows just above the horizon
-                                   first; the sun-cone taps of a sample are fetched one at a time in
-                                   full frames, in pairs in large 1/16-pixel launches and all six
-                                   together in launches of <= 262144 rays (latency-bound) */
+                                   first, the sun cones deferred and computed 32 at a time; launches of
+                                   <= 600000 rays, bound by their longest rays, give each ray a team of
+                                   2, 4 or 8 lanes instead */
     MM_SCHEDULE_PERSISTENT = 1  /* persistent warps; each iteration evaluates one cloudTest per lane
                                    (a march step or a sun-cone tap); finished lanes take the next ray
                                    of their warp's 8x4 pixel tile (ballot compaction).  Full SIMT
@@ -422,8 +422,8 @@ typedef struct mm_view {
 typedef enum mm_batch_schedule {
     MM_BATCH_PERSISTENT = 0, /* persistent warps take warp tiles of all views from one global queue */
     MM_BATCH_BLOCKS = 1,     /* one launch of 16x8-pixel blocks over all views, hardware-scheduled */
-    MM_BATCH_GRAPH = 2       /* one CUDA graph of the views' own launches (each view's kernel variant) on
-                                four concurrent branches, largest views first */
+    MM_BATCH_GRAPH = 2       /* one CUDA graph of the views' own launches (the kernel variant that suits
+                                the rays of all of them) on four concurrent branches, largest views first */
 } mm_batch_schedule;
 
 typedef struct mm_batch_options {

@@ -173,6 +173,8 @@ int capture_views(mm_context ctx, BatchState* b, const mm_view* views, int n, co
         }
         order[j + 1] = v;
     }
+    long long rays = 0;  // of all views: they run side by side
+    for (int i = 0; i < n; ++i) rays += (long long)views[i].out.width * views[i].out.height;
     int r = MM_OK;
     cudaError_t e = cudaStreamBeginCapture(b->branch[0], cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
@@ -195,7 +197,8 @@ int capture_views(mm_context ctx, BatchState* b, const mm_view* views, int n, co
             r = mm::launch_surrogate_frame(p, ctx, o.surrogate, b->branch[0]);
         else
             r = mm::launch_march_fast(p, MM_SAMPLER_HARDWARE, o.density_format, MM_SCHEDULE_TILED, 0, ctx->d_work,
-                                      ctx->num_sms, b->branch[o.surrogate ? 0 : i % K]);
+                                      ctx->num_sms, b->branch[o.surrogate ? 0 : i % K],
+                                      o.surrogate ? 0 : rays - (long long)v.out.width * v.out.height);
     }
     for (int k = 1; k < K; ++k) {
         cudaEventRecord(b->join[k], b->branch[k]);

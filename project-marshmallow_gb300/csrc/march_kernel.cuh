@@ -947,48 +947,8 @@ __device__ __forceinline__ int tile_py(int by, int warp, int lane) {
     return by * kBlockTileH + (warp / kWarpsAcross) * kWarpTileH + lane / kWarpTileW;
 }
 
-// Three variants of the same march, chosen per launch:
-//  - full frames: one cone tap at a time (G = 1) keeps registers low enough for 10 blocks per SM,
-//    and the texture unit is kept busy by the many warps;
-//  - launches of at most kLatencyRays rays (a 1920x1080 frame at 1/16 of its pixels, or a small
-//    image): such a launch is bounded below by the latency of its longest rays (a few hundred
-//    dependent samples just above the horizon, ~0.5 ms on GB300 whatever the launch size), so all
-//    six sun-cone taps of a sample are issued together (G = 6: a sample's cone takes 3 dependent
-//    fetch rounds instead of up to 18) at 3 blocks per SM for the registers;
-//  - larger 1/16-pixel launches (3840x2160/16: several waves): cone taps in threes (G = 3, 6 blocks).
-// Measured over the 16-frame sweep (mean of frames 0, 5, 10, 15; production units built with
-// denormals flushed): 1920x1080/16 0.48 ms (G = 6); 3840x2160/16 0.68 (G = 1, 10 blocks), 0.56
-// (G = 2, 7 or 8 blocks), 0.53 (G = 3, 6 blocks), 0.54 / 0.56 (G = 3, 5 / 7 blocks), 0.60 / 0.67
-// (G = 6, 4 / 3 blocks).  Both small-launch variants issue a small-step sample's curl fetch ahead of
-// its cloudTest fetches (SC): the longest rays are chains of small-step samples whose density is then
-// eroded away by cloudHiRes (~170 of their ~700 dependent fetch rounds), and SC takes one round out
-// of each: 1920x1080/16 0.35 -> 0.32 ms, 3840x2160/16 0.42 -> 0.41 ms.  Full frames, bound by
-// throughput, lose by the wasted fetches (3.24 -> 3.28 ms) and keep it off.
 #ifndef MM_TILED_PARAM_CONE
 #define MM_TILED_PARAM_CONE 0  // full frames: cone offsets from the launch parameters, cone loop unrolled
-#endif
-#ifndef MM_PHASE16_CONE_GROUP
-#define MM_PHASE16_CONE_GROUP 3
-#endif
-#ifndef MM_PHASE16_MIN_BLOCKS
-#define MM_PHASE16_MIN_BLOCKS 6
-#endif
-#ifndef MM_PHASE16_SPEC_CURL
-#define MM_PHASE16_SPEC_CURL 1
-#endif
-#ifndef MM_LATENCY_SPEC_CURL
-#define MM_LATENCY_SPEC_CURL 1
-#endif
-#ifndef MM_LATENCY_MIN_BLOCKS
-#define MM_LATENCY_MIN_BLOCKS 3
-#endif
-
-#ifndef MM_LATENCY_RAYS
-#define MM_LATENCY_RAYS 262144
-#endif
-constexpr long long kLatencyRays = MM_LATENCY_RAYS;
-#ifndef MM_LATENCY_SCHEDULE
-#define MM_LATENCY_SCHEDULE 1  // launches of at most kLatencyRays rays: 1 = team march, 0 = one thread per ray
 #endif
 
 template <bool E, int S, bool C, int G, bool SC, bool PC = false, int LP = 0>
@@ -1048,17 +1008,6 @@ constexpr int kPool = 64;  // records per warp: < 32 after a round, + at most 32
 // 1920x1080 sweeps: 3.184 / 0.986 ms against 3.212 / 0.992 (fewer spills: 64 B against 72 B).
 #ifndef MM_POOL_PARAM_CONE
 #define MM_POOL_PARAM_CONE 1
-#endif
-// 1/16-pixel launches above kLatencyRays rays: pooled cones (1) or the inline kernel with cone taps in
-// threes at 6 blocks per SM (0).  3840x2160 at 1/16, sweep frames 0/5/10/15: 0.361 against 0.412 ms.
-#ifndef MM_PHASE16_POOL
-#define MM_PHASE16_POOL 1
-#endif
-// The team march's one-thread rows: pooled cones (1) or inline cone taps in threes (0).  1920x1080 at
-// 1/16, sweep mean: 0.256 ms pooled against 0.247 (the launch is bound by its longest rays, which the
-// teams march; the pool's rounds only add latency to the others).
-#ifndef MM_HYBRID_POOL
-#define MM_HYBRID_POOL 0
 #endif
 struct ConePool {
     float t[MM_TILED_WARPS][kPool], step[MM_TILED_WARPS][kPool], acc[MM_TILED_WARPS][kPool];
@@ -1274,16 +1223,6 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PAIR_MIN_BLOCKS) march
     march_tiled_body<false, MM_SAMPLER_HARDWARE, C, MM_CONE_GROUP, (MM_SPEC_CURL != 0), (MM_TILED_PARAM_CONE != 0), 2>(p);
 }
 
-template <bool E, int S, bool C>
-__global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PHASE16_MIN_BLOCKS) march_tiled_phase16_kernel(MarchLaunch p) {
-    march_tiled_body<E, S, C, MM_PHASE16_CONE_GROUP, (MM_PHASE16_SPEC_CURL != 0), true>(p);
-}
-
-template <bool E, int S, bool C>
-__global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_LATENCY_MIN_BLOCKS) march_tiled_latency_kernel(MarchLaunch p) {
-    march_tiled_body<E, S, C, 6, (MM_LATENCY_SPEC_CURL != 0), true>(p);
-}
-
 // ------------------------------------------------------------------------------ team march
 //
 // Launches of few rays (a 1920x1080 frame at 1/16 of its pixels) are bound by the chain of
@@ -1293,40 +1232,73 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_LATENCY_MIN_BLOCKS) ma
 // reach j iterations later if nothing changed the step size or the mode: position t + s + ... + s
 // (j additions, as the loop's increments make it), its cloudTest, and in small-step mode its
 // cloudHiRes, sun cone and shading term where the shader would compute them.  The team then runs
-// the loop body (:408-482) sample by sample in order on the shuffled results, every member the
-// same state; a step back (:426-434) or a return to large steps (:468-474) changes the step size,
-// so the rest of the round is dropped and the next round starts where the loop goes on.  Every
-// consumed sample is the computation the sequential loop does, in the same arithmetic, so the
-// output (and the work counts, which count consumed samples only) equals the one-thread march.
-#ifndef MM_TEAM_LANES
-#define MM_TEAM_LANES 4
+// the loop body (:408-482) on the round's results in order, every member the same state; a step back
+// (:426-434) or a return to large steps (:468-474) changes the step size, so the rest of the round is
+// dropped and the next round starts where the loop goes on.  Every consumed sample is the computation
+// the sequential loop does, in the same arithmetic, so the output (and the work counts, which count
+// consumed samples only) equals the one-thread march.
+//
+// Which launches take teams, and of how many lanes.  A launch takes at least as long as its longest
+// rays, ~300 us one thread per ray; a team of n lanes makes that chain shorter, but costs lanes: each
+// member sets the ray up, and a round's tail is dropped at every step-size change.  The more rays, the
+// smaller the teams; past ~600,000 rays the pooled kernel's throughput wins.  Cone taps in groups of G
+// at B blocks per SM: a larger G is faster for a ray, a larger B for the launch.  Microseconds on GB300,
+// pitch 12, two seeds, whole images and (f) frames with 1 pixel in 16 marched (the reprojection beside):
+//   rays         36k    65k    76k    90k   153k   256k   331k   412k   518k   589k  704k   f129k  f518k
+//   8 G3 B6     71.8   82.7  100.0  118.1  171.9  268.2  338.6  414.9  508.2  570.1  664.8  175.2  600.3
+//   4 G3 B6    107.8  110.0  118.7  117.6  147.3  223.0  276.0  334.6  406.7  452.5  525.6  155.7  491.3
+//   4 G3 B7    111.5  113.4  122.7  122.3  142.7  214.1  264.7  320.3  389.3  432.9  502.7  155.3  473.8
+//   2 G2 B7    198.5  209.2  221.0  207.5  212.7  214.2  250.2  295.9  351.3  387.2  438.8  241.5  421.7
+//   2 G2 B8    222.7  231.4  243.4  227.6  235.7  234.4  255.3  295.2  349.6  384.8  434.9  264.2  417.3
+//   pooled     276.3  294.2  301.2  272.4  294.2  297.6  304.0  320.0  384.7  421.0  361.9  369.4  456.7
+// Launches that run side by side (the views of a batch) fill the GPU together, so their rays together
+// decide: six 512x512 faces and six cameras of 535,000 to 922,000 rays in one call take 2783 us with
+// each view's own choice and 2403 us with all of them pooled.  4 G3 stays at 6 blocks though 7 is 3%
+// faster above 150,000 rays: at 7 the compiler contracts other products, and the team sizes would no
+// longer agree to the last bit.  (2 G1 at 8 to 10 blocks, 4 G2 B8, 8 G2 B7 and 8 G3 B5 are slower everywhere or within 1%.)
+#ifndef MM_TEAM8_RAYS
+#define MM_TEAM8_RAYS 90000
 #endif
-#ifndef MM_TEAM_MIN_BLOCKS
-#define MM_TEAM_MIN_BLOCKS 4
+#ifndef MM_TEAM4_RAYS
+#define MM_TEAM4_RAYS 262144
 #endif
-// Cone taps a team member issues together (6 or 3).  1920x1080/16 sweep mean, 256x256: taps in
-// sixes at 4 blocks/SM (127 registers) 0.247 / 0.160 ms; in threes at 5 / 6 / 8 blocks/SM 0.256 /
-// 0.282 / 0.321 and 0.163 / 0.179 / 0.189; sixes at 5 blocks/SM (96 registers) 0.256 / 0.169.
-#ifndef MM_TEAM_CONE_GROUP
-#define MM_TEAM_CONE_GROUP 6
+#ifndef MM_TEAM2_RAYS
+#define MM_TEAM2_RAYS 600000
 #endif
-constexpr int kTeam = MM_TEAM_LANES;
-static_assert(kTeam == 4 || kTeam == 8, "team size");
-// Rays of a warp (32 / kTeam) as a 2x2 (teams of 8) or 4x2 (teams of 4) pixel tile; the four warps
-// of a block side by side in a 2x2 arrangement.
-constexpr int kTeamWarpW = kTeam == 8 ? 2 : 4, kTeamWarpH = 2;
-constexpr int kTeamBlockW = 2 * kTeamWarpW, kTeamBlockH = 2 * kTeamWarpH;
+constexpr long long kTeam8Rays = MM_TEAM8_RAYS, kTeam4Rays = MM_TEAM4_RAYS, kTeam2Rays = MM_TEAM2_RAYS;
+constexpr long long kHalf2Rays = 262144;  // MM_MATH_FAST_HALF2: images up to here take teams (FP32 decisions)
 
-// One ray marched by the calling team (member `member` of the kTeam lanes at `base` of the warp).
-template <bool E, int S, bool C>
+// A team of kT lanes; the rays of a warp (32 / kT) as a pixel tile, the four warps of a block side by
+// side in a 2x2 arrangement.
+template <int kT>
+struct TeamTile {
+    static_assert(kT == 2 || kT == 4 || kT == 8, "team size");
+    static constexpr int kWarpW = kT == 8 ? 2 : 4, kWarpH = 32 / kT / kWarpW;
+    static constexpr int kBlockW = 2 * kWarpW, kBlockH = 2 * kWarpH;
+};
+
+// One ray marched by the calling team (member `member` of the kTeam lanes at `base` of the warp; G cone taps
+// issued together).  Every
+// lane of the warp calls it and stays until the last team is done (`inside` = false: a team without a
+// pixel), so the round's results are exchanged by full-warp ballots: three ballots tell every member
+// which samples are valid, hit, and accumulate, and the loop state follows from the bits.  Only a
+// round in which some team of the warp accumulates shuffles values.  Taking the loop body sample by
+// sample on shuffled results instead (up to 16 shuffles under per-team masks a round) made the resolve
+// two fifths of the round: 256x256, teams of 4 with cone taps in sixes at 4 blocks per SM, 147.7 -> 92.8 us.
+template <bool E, int S, bool C, int kTeam, int G>
 __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, const V3* s_cone, int px, int py,
-                                         int member, int base, unsigned tmask) {
+                                         bool inside, int member, int base) {
+    const unsigned full = 0xffffffffu;
     Work w;
-    const Ray r = ray_setup<E, S>(p, f, px, py);
-    if (r.killed) {
-        if (member == 0) store_pixel(p, px, py, make_float4(r.bg.x, r.bg.y, r.bg.z, r.alpha), CUDART_INF_F);
-        return;
+    Ray r{};
+    bool done = true;
+    if (inside) {
+        r = ray_setup<E, S>(p, f, px, py);
+        done = r.killed;
+        if (r.killed && member == 0)
+            store_pixel(p, px, py, make_float4(r.bg.x, r.bg.y, r.bg.z, r.alpha), CUDART_INF_F);
     }
+    const bool live = !done;
     const V3 rd = r.rd;
     float accum = 0.0f, transmittance = 1.0f;
     float stepSize = 0.05f * f.thickness;  // :390
@@ -1334,12 +1306,17 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
     int misses = 0, steps = 0, iterations = 0;
     float firstT = CUDART_INF_F;
     float t = r.t0;
-    bool done = false;
-    while (!done) {
-        // ---- this member's sample of the round
+    while (__any_sync(full, !done)) {
+        // ---- the round's positions (the loop's own additions) and this member's sample
+        float ts[kTeam];
+        ts[0] = t;
         float tj = t;
-        for (int k = 0; k < member; ++k) tj += stepSize;
-        const bool valid = tj < r.t1 && iterations + member < kMaxIterations;
+#pragma unroll
+        for (int k = 1; k < kTeam; ++k) {
+            ts[k] = ts[k - 1] + stepSize;
+            if (member == k) tj = ts[k];
+        }
+        const bool valid = !done && tj < r.t1 && iterations + member < kMaxIterations;
         float lo = 0.0f, hi = 0.0f, y = 0.0f;
         unsigned long long nt = 0, nh = 0;
         if (valid) {
@@ -1352,110 +1329,147 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                 hi = hires_finish<E>(hires_fetch<E, S>(p, curl_displace<E>(g, stepSize, cu)), g.rh, lo, nh);
                 if (hi >= 0.0001f) {
                     float dal = 0.0f;
+                    if constexpr (!E) {
 #pragma unroll
-                    for (int i = 0; i < 6; i += MM_TEAM_CONE_GROUP)
-                        dal = cone_taps<E, S, MM_TEAM_CONE_GROUP, true>(p, f, s_cone, i, pos, stepSize, dal, nt, nh);
+                        for (int i = 0; i < 6; i += G)
+                            dal = cone_taps<E, S, G, true>(p, f, s_cone, i, pos, stepSize, dal, nt, nh);
+                    } else {
+#pragma unroll 1
+                        for (int i = 0; i < 6; i += G)
+                            dal = cone_taps<E, S, G>(p, f, s_cone, i, pos, stepSize, dal, nt, nh);
+                    }
                     y = shade_term<E>(dal, lo, g.rh, r.cosTheta, r.hg);
                 }
             }
         }
-        // ---- the loop body (:408-482) on the round's samples, in order
-#pragma unroll 1
-        for (int i = 0; i < kTeam; ++i) {
-            const bool vi = __shfl_sync(tmask, valid, base + i);
-            if (!vi) {  // the loop condition fails at this iteration: the ray is finished
-                done = true;
-                break;
+        constexpr unsigned kMask = (1u << kTeam) - 1u;
+        const unsigned vb = (__ballot_sync(full, valid) >> base) & kMask;
+        const unsigned hb = (__ballot_sync(full, lo > 0.0f) >> base) & kMask;
+        const unsigned kept = __ballot_sync(full, hi >= 0.0001f);
+        const int n = __ffs(~vb) - 1;  // valid samples: the first n
+        int used = 0;                  // samples the loop consumes this round
+        bool turn = false, back = false;
+        if (!C && kept == 0u) {
+            // ---- no team accumulates: the loop body (:408-482) on the bits alone
+            const int lead = hb ? __ffs(hb) - 1 : n;  // samples without density before the first hit
+            int counted;
+            if (noHits) {
+                turn = hb != 0u;
+                used = turn ? lead + 1 : n;
+                counted = lead;
+            } else {
+                back = misses + lead >= 10;  // :468-474; a run after a hit is shorter than 10
+                used = back ? 10 - misses : n;
+                counted = __popc(~hb & ((1u << used) - 1u));
+                misses = hb ? n - (32 - __clz(hb)) : misses + n;
             }
-            const float li = __shfl_sync(tmask, lo, base + i);
-            const float hiv = __shfl_sync(tmask, hi, base + i);
-            const float yi = __shfl_sync(tmask, y, base + i);
-            if (C) {
-                w.test += (unsigned)__shfl_sync(tmask, (unsigned)nt, base + i);
-                w.hires += (unsigned)__shfl_sync(tmask, (unsigned)nh, base + i);
-            }
-            ++w.iter;
-            bool restart = false;
-            if (li > 0.0f) {
-                misses = 0;
-                if (noHits) {  // :428-434: back half a step, small steps from here
-                    t -= stepSize;
-                    stepSize *= 0.3f;
-                    noHits = false;
-                    restart = true;
-                } else if (hiv >= 0.0001f) {  // :437-466
-                    transmittance = mixf(transmittance, yi, 1.0f - accum);
-                    ++w.acc;
-                    if (firstT == CUDART_INF_F) firstT = t;
-                    accum += hiv;
+            steps += counted;
+            if (steps > 100) done = true;                          // :481
+            if (!turn && !back && n < kTeam) done = true;          // the loop condition (:408)
+        } else {
+            // ---- the loop body sample by sample on the exchanged results
+            const unsigned kb = (kept >> base) & kMask;
+            bool run = !done;
+#pragma unroll
+            for (int i = 0; i < kTeam; ++i) {
+                const float hiv = __shfl_sync(full, hi, base + i);
+                const float yi = __shfl_sync(full, y, base + i);
+                unsigned ti = 0, hn = 0;
+                if (C) {
+                    ti = __shfl_sync(full, (unsigned)nt, base + i);
+                    hn = __shfl_sync(full, (unsigned)nh, base + i);
+                }
+                if (run && !((vb >> i) & 1u)) {  // the loop condition fails: the ray is finished
+                    done = true;
+                    run = false;
+                }
+                if (run) {
+                    ++used;
+                    if (C) {
+                        ++w.iter;
+                        w.test += ti;
+                        w.hires += hn;
+                    }
+                    bool count = false;
+                    if ((hb >> i) & 1u) {
+                        misses = 0;
+                        if (noHits) {  // :428-434
+                            turn = true;
+                        } else if ((kb >> i) & 1u) {  // :437-466
+                            transmittance = mixf(transmittance, yi, 1.0f - accum);
+                            if (C) ++w.acc;
+                            if (firstT == CUDART_INF_F) firstT = ts[i];
+                            accum += hiv;
+                            count = true;
+                        }
+                    } else {
+                        if (!noHits) {  // :468-474
+                            misses++;
+                            back = misses >= 10;
+                        }
+                        count = true;
+                    }
                     if (accum > 0.99f) {  // :476-479
                         accum = 1.0f;
                         done = true;
-                        break;
-                    }
-                    if (++steps > 100) {
+                    } else if (count && ++steps > 100) {  // :481
                         done = true;
-                        break;
                     }
-                }
-            } else {
-                if (!noHits) {  // :468-474
-                    misses++;
-                    if (misses >= 10) {
-                        noHits = true;
-                        stepSize = M<E>::div(stepSize, 0.3f);
-                        restart = true;
-                    }
-                }
-                if (++steps > 100) {  // :481
-                    done = true;
-                    break;
+                    run = !(done || turn || back);
                 }
             }
-            t += stepSize;  // the loop increment (:408), also after a `continue`
-            ++iterations;
-            if (restart) break;
         }
+        // ---- on to the next round: the increment (:408), after a step back half a step (:428-434)
+        // or a return to large steps
+        iterations += used;
+#pragma unroll
+        for (int k = 0; k < kTeam; ++k)
+            if (used == k + 1) t = ts[k];
+        if (turn) {
+            misses = 0;
+            t -= stepSize;
+            stepSize *= 0.3f;
+            noHits = false;
+        }
+        if (back) {
+            noHits = true;
+            stepSize = M<E>::div(stepSize, 0.3f);
+        }
+        t += stepSize;
     }
-    if (member == 0) {
+    if (live && member == 0) {
         store_pixel(p, px, py, composite<E>(p.u, f, r.rd, r.bg, r.alpha, accum, transmittance), firstT);
         if (C) flush_work(p.counters, w);
     }
 }
 
-// Band of ray rows marched by teams, the rest one thread per ray, in one launch: the first
-// team_blocks blocks march kTeamBlockW x kTeamBlockH ray tiles of the band [band0, band1) from its
-// bottom row (the horizon) up, the others 16 x 8 tiles of the rows above the band (nearest first)
-// and then of the rows below it (rays under the horizon, which end at once).
-struct HybridGrid {
-    int team_bx, team_blocks;  // team tiles per band row, team blocks in all
-    int band0, band1;          // ray rows [band0, band1), multiples of 8
-    int single_bx;             // 16-wide tiles per row
-    int rows_above;            // 8-row block rows above the band
+// One launch: the first team_blocks blocks march the ray rows above the horizon by teams, from the
+// horizon (the longest rays) up; the others take the rows below it, whose rays end at once, one thread
+// per ray in 16 x 8 tiles.
+struct TeamGrid {
+    int team_bx, team_blocks;  // team tiles per row of tiles, team blocks in all
+    int horizon;               // ray rows [0, horizon) by teams, a multiple of 8
+    int single_bx;             // 16-wide tiles per row below
 };
 
-template <bool E, int S, bool C>
-__global__ void __launch_bounds__(128, MM_TEAM_MIN_BLOCKS) march_hybrid_kernel(MarchLaunch p, HybridGrid hg) {
+template <bool E, int S, bool C, int kTeam, int G, int kMinBlocks>
+__global__ void __launch_bounds__(128, kMinBlocks) march_team_kernel(MarchLaunch p, TeamGrid tg) {
     __shared__ V3 s_cone[6];
-#if MM_HYBRID_POOL
-    __shared__ ConePool s_q;
-#endif
     cone_offsets(p.u, s_cone);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int tx, ty;
-    const bool team_block = (int)blockIdx.x < hg.team_blocks;
+    const bool team_block = (int)blockIdx.x < tg.team_blocks;
     if (team_block) {
-        const int bx = (int)blockIdx.x % hg.team_bx, byr = (int)blockIdx.x / hg.team_bx;
+        using T = TeamTile<kTeam>;
+        const int bx = (int)blockIdx.x % tg.team_bx, byr = (int)blockIdx.x / tg.team_bx;
         const int team = lane / kTeam;
-        tx = bx * kTeamBlockW + (warp & 1) * kTeamWarpW + team % kTeamWarpW;
-        ty = hg.band1 - kTeamBlockH * (byr + 1) + (warp >> 1) * kTeamWarpH + team / kTeamWarpW;
+        tx = bx * T::kBlockW + (warp & 1) * T::kWarpW + team % T::kWarpW;
+        ty = tg.horizon - T::kBlockH * (byr + 1) + (warp >> 1) * T::kWarpH + team / T::kWarpW;
     } else {
-        const int idx = (int)blockIdx.x - hg.team_blocks;
-        const int bx = idx % hg.single_bx, k = idx / hg.single_bx;
-        const int row0 = k < hg.rows_above ? hg.band0 - 8 * (k + 1) : hg.band1 + 8 * (k - hg.rows_above);
-        tx = bx * 16 + (warp & 1) * 8 + (lane & 7);
-        ty = row0 + (warp >> 1) * 4 + (lane >> 3);
+        const int idx = (int)blockIdx.x - tg.team_blocks;
+        tx = idx % tg.single_bx * 16 + (warp & 1) * 8 + (lane & 7);
+        ty = tg.horizon + idx / tg.single_bx * 8 + (warp >> 1) * 4 + (lane >> 3);
     }
     int px, py;
     if (p.pixel_mode == MM_PIXELS_PHASE16) {  // :292-298
@@ -1466,80 +1480,40 @@ __global__ void __launch_bounds__(128, MM_TEAM_MIN_BLOCKS) march_hybrid_kernel(M
         py = ty;
     }
     const bool inside = px < p.width && py < p.height;
-#if MM_HYBRID_POOL
-    if (!team_block) {  // every lane of the warp stays: the pool's rounds need them all
-        const Frame f = make_frame<E>(p);
-        Work w;
-        march_pixel_q<E, S, (MM_SPEC_CURL != 0)>(p, f, s_cone, s_q, px, py, inside, w);
-        if (C) flush_work(p.counters, w);
-        return;
-    }
-#endif
-    if (!inside) return;  // a team leaves together: its lanes share (px, py)
     const Frame f = make_frame<E>(p);
-    if (team_block) {
-        const int team = lane / kTeam, base = team * kTeam;
-        team_ray<E, S, C>(p, f, s_cone, px, py, lane % kTeam, base, ((1u << kTeam) - 1u) << base);
-    } else {
+    if (team_block) {  // every lane of the warp stays: the rounds' ballots need them all
+        team_ray<E, S, C, kTeam, G>(p, f, s_cone, px, py, inside, lane % kTeam, lane / kTeam * kTeam);
+    } else if (inside) {
         Work w;
-        march_pixel<E, S, 3, true, true>(p, f, s_cone, px, py, w);
+        march_pixel<E, S>(p, f, s_cone, px, py, w);
         if (C) flush_work(p.counters, w);
     }
 }
 
-// The band for a launch: ray rows whose rays rise at less than MM_TEAM_BAND_DEG degrees (the long
-// ones: at 6 degrees a ray crosses ~190 km of the shell and hits the 100-step limit), widened to
-// multiples of 8 rows and running down to the horizon; a launch of at most MM_TEAM_ALL_RAYS rays
-// marches every row above the horizon by teams.  Empty for a camera with roll (right.y != 0: a
-// row's rays then rise at different angles).  Measured over the 16-frame sweep on GB300, mean
-// ms per launch, against 0.308 (1920x1080 at 1/16) and 0.312 (256x256) one thread per ray:
-//   band 6 deg 0.246 / 0.224, 12 deg 0.264 / 0.193, 25 deg 0.261 / 0.175, every row 0.298 / 0.160.
-// A launch of one wave or less gains from teams everywhere; in a larger one the teams' extra
-// lanes cost more than they save on rays that are not the longest.
-#ifndef MM_TEAM_BAND_DEG
-#define MM_TEAM_BAND_DEG 6
-#endif
-#ifndef MM_TEAM_ALL_RAYS
-#define MM_TEAM_ALL_RAYS 65536
-#endif
-inline HybridGrid hybrid_grid(const MarchLaunch& p, int gw, int gh) {
-    HybridGrid g{};
-    const int ghp = (gh + 7) / 8 * 8;
-    int band0 = ghp, band1 = ghp;
+// The ray rows above the horizon, rounded up to 8: for a camera without roll (right.y == 0) a row's
+// rays all rise or all fall; any other camera marches every row by teams.
+template <int kTeam>
+TeamGrid team_grid(const MarchLaunch& p, int gw, int gh) {
+    TeamGrid g{};
+    int horizon = gh;
     const float* v = p.u.camera.view;
     if (v[4] == 0.0f) {
         const double cpy = p.u.camera.camera_params[1];
-        const double lx = v[2], ly = v[6], lz = v[10], ux = v[1], uy = v[5], uz = v[9];
-        const double s_band = (long long)gw * gh <= MM_TEAM_ALL_RAYS
-                                  ? 2.0
-                                  : sin((double)MM_TEAM_BAND_DEG * 3.14159265358979323846 / 180.0);
         const bool phase16 = p.pixel_mode == MM_PIXELS_PHASE16;
-        int first = -1, horizon = gh;
         for (int ty = 0; ty < gh; ++ty) {
             const int py = phase16 ? ty * 4 + p.phase / 4 : ty;
-            const double sy = 2.0 * py / p.uv_h - 1.0;
-            // centre-column ray direction (compute-clouds.comp:309-322): -look - sy * tan * up
-            const double dx = -lx - sy * cpy * ux, dy = -ly - sy * cpy * uy, dz = -lz - sy * cpy * uz;
-            const double sin_el = dy / sqrt(dx * dx + dy * dy + dz * dz);
-            if (sin_el <= 0.0) {
+            // y of the row's ray directions (compute-clouds.comp:309-322): -look - sy * tan * up
+            if (-(double)v[6] - (2.0 * py / p.uv_h - 1.0) * cpy * v[5] <= 0.0) {
                 horizon = ty;
                 break;
             }
-            if (first < 0 && sin_el < s_band) first = ty;
-        }
-        if (first >= 0 && first < horizon) {
-            band0 = first / 8 * 8;
-            band1 = (horizon + 7) / 8 * 8;
-            if (band1 > ghp) band1 = ghp;
         }
     }
-    if (band0 >= band1) band0 = band1 = ghp;  // no band: every row one thread per ray
-    g.band0 = band0;
-    g.band1 = band1;
-    g.team_bx = (gw + kTeamBlockW - 1) / kTeamBlockW;
-    g.team_blocks = g.team_bx * ((band1 - band0) / kTeamBlockH);
+    using T = TeamTile<kTeam>;
+    g.horizon = (horizon + 7) / 8 * 8;
+    g.team_bx = (gw + T::kBlockW - 1) / T::kBlockW;
+    g.team_blocks = g.team_bx * (g.horizon / T::kBlockH);
     g.single_bx = (gw + 15) / 16;
-    g.rows_above = band0 / 8;
     return g;
 }
 
@@ -1613,8 +1587,20 @@ void prepare_march_kernels() {
     pool_carveout<E, MM_SAMPLER_SOFTWARE, true>();
 }
 
+template <bool E, int S, int kTeam, int G, int kMinBlocks>
+void launch_team(const MarchLaunch& p, int gw, int gh, cudaStream_t s) {
+    const TeamGrid tg = team_grid<kTeam>(p, gw, gh);
+    const int rows = (gh + 7) / 8 * 8;
+    const int blocks = tg.team_blocks + tg.single_bx * ((rows - tg.horizon) / 8);
+    if (p.counters)
+        march_team_kernel<E, S, true, kTeam, G, kMinBlocks><<<blocks, 128, 0, s>>>(p, tg);
+    else
+        march_team_kernel<E, S, false, kTeam, G, kMinBlocks><<<blocks, 128, 0, s>>>(p, tg);
+}
+
+// beside: rays of the other launches that run at the same time (0: this one has the GPU to itself).
 template <bool E, int S>
-int launch_tiled(const MarchLaunch& p0, cudaStream_t s, bool half2 = false) {
+int launch_tiled(const MarchLaunch& p0, cudaStream_t s, bool half2 = false, long long beside = 0) {
     MarchLaunch p = p0;
     int gw = p.width, gh = p.height;
     if (p.pixel_mode == MM_PIXELS_PHASE16) {
@@ -1626,29 +1612,16 @@ int launch_tiled(const MarchLaunch& p0, cudaStream_t s, bool half2 = false) {
     // Kernels that the build knobs leave unused are not instantiated (if constexpr).
     const bool C = p.counters != nullptr;
     const dim3 block(MM_TILED_WARPS * 32);
-    if ((long long)gw * gh <= kLatencyRays) {
-        if constexpr (MM_LATENCY_SCHEDULE == 1) {
-            const HybridGrid hg = hybrid_grid(p, gw, gh);
-            const int blocks =
-                hg.team_blocks + hg.single_bx * (hg.rows_above + ((gh + 7) / 8 * 8 - hg.band1) / 8);
-            if (C)
-                march_hybrid_kernel<E, S, true><<<blocks, 128, 0, s>>>(p, hg);
-            else
-                march_hybrid_kernel<E, S, false><<<blocks, 128, 0, s>>>(p, hg);
-        } else {
-            if (C)
-                march_tiled_latency_kernel<E, S, true><<<grid, block, 0, s>>>(p);
-            else
-                march_tiled_latency_kernel<E, S, false><<<grid, block, 0, s>>>(p);
-        }
-    } else if (p.pixel_mode == MM_PIXELS_PHASE16 && !MM_PHASE16_POOL) {
-        if constexpr (!MM_PHASE16_POOL) {
-            if (C)
-                march_tiled_phase16_kernel<E, S, true><<<grid, block, 0, s>>>(p);
-            else
-                march_tiled_phase16_kernel<E, S, false><<<grid, block, 0, s>>>(p);
-        }
-    } else if (!E && S == MM_SAMPLER_HARDWARE && half2 && p.pixel_mode != MM_PIXELS_PHASE16) {
+    const long long rays = (long long)gw * gh + beside;
+    const bool h2 = !E && S == MM_SAMPLER_HARDWARE && half2 && p.pixel_mode != MM_PIXELS_PHASE16;
+    if (rays <= (h2 ? kHalf2Rays : kTeam2Rays)) {
+        if (rays <= kTeam8Rays)
+            launch_team<E, S, 8, E ? 1 : 3, E ? 3 : 6>(p, gw, gh, s);
+        else if (rays <= kTeam4Rays)
+            launch_team<E, S, 4, E ? 1 : 3, E ? 3 : 6>(p, gw, gh, s);
+        else
+            launch_team<E, S, 2, E ? 1 : 2, E ? 3 : 7>(p, gw, gh, s);
+    } else if (h2) {
         if constexpr (!E && S == MM_SAMPLER_HARDWARE) {
             if (C)
                 march_tiled_h2_kernel<true><<<grid, block, 0, s>>>(p);

@@ -109,8 +109,9 @@ void prepare_march_exact_sw();
 int launch_march_exact_sw(const MarchLaunch& p, int schedule, unsigned int* work, int num_sms, cudaStream_t s);
 int launch_march_exact(const MarchLaunch& p, int sampler, int schedule, unsigned int* work, int num_sms,
                        cudaStream_t s);
+// beside: rays of the other launches that run at the same time (the other views of a batch).
 int launch_march_fast(const MarchLaunch& p, int sampler, int format, int schedule, int half2, unsigned int* work,
-                      int num_sms, cudaStream_t s);
+                      int num_sms, cudaStream_t s, long long beside = 0);
 
 // Noise generators (noise.cu).
 int launch_noise(int kind, uint32_t seed, int w, int h, int d, uint8_t* out, cudaStream_t s);
