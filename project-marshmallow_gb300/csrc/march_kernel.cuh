@@ -1252,8 +1252,8 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PAIR_MIN_BLOCKS) march
 //   2 G2 B8    222.7  231.4  243.4  227.6  235.7  234.4  255.3  295.2  349.6  384.8  434.9  264.2  417.3
 //   pooled     276.3  294.2  301.2  272.4  294.2  297.6  304.0  320.0  384.7  421.0  361.9  369.4  456.7
 // Launches that run side by side (the views of a batch) fill the GPU together, so their rays together
-// decide: six 512x512 faces and six cameras of 535,000 to 922,000 rays in one call take 2783 us with
-// each view's own choice and 2403 us with all of them pooled.  4 G3 stays at 6 blocks though 7 is 3%
+// decide: six 512x512 faces and six cameras of 535,000 to 922,000 rays in one call take 2612 us with
+// each view's own choice and 2273 us with half the others' rays counted to its own (batch.cu).  4 G3 stays at 6 blocks though 7 is 3%
 // faster above 150,000 rays: at 7 the compiler contracts other products, and the team sizes would no
 // longer agree to the last bit.  (2 G1 at 8 to 10 blocks, 4 G2 B8, 8 G2 B7 and 8 G3 B5 are slower everywhere or within 1%.)
 #ifndef MM_TEAM8_RAYS
@@ -1502,8 +1502,10 @@ TeamGrid team_grid(const MarchLaunch& p, int gw, int gh) {
         const bool phase16 = p.pixel_mode == MM_PIXELS_PHASE16;
         for (int ty = 0; ty < gh; ++ty) {
             const int py = phase16 ? ty * 4 + p.phase / 4 : ty;
-            // y of the row's ray directions (compute-clouds.comp:309-322): -look - sy * tan * up
-            if (-(double)v[6] - (2.0 * py / p.uv_h - 1.0) * cpy * v[5] <= 0.0) {
+            // y of the row's ray directions (compute-clouds.comp:309-322): -look - sy * tan * up.  A row
+            // that runs level is marched (only rd.y < 0 is not, :351) and has the longest rays of all,
+            // so the line lies below what the kernel's rounding can take for level.
+            if (-(double)v[6] - (2.0 * py / p.uv_h - 1.0) * cpy * v[5] < -1.0e-5) {
                 horizon = ty;
                 break;
             }
