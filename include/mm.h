@@ -422,8 +422,8 @@ typedef struct mm_view {
 typedef enum mm_batch_schedule {
     MM_BATCH_PERSISTENT = 0, /* persistent warps take warp tiles of all views from one global queue */
     MM_BATCH_BLOCKS = 1,     /* one launch of 16x8-pixel blocks over all views, hardware-scheduled */
-    MM_BATCH_GRAPH = 2       /* one CUDA graph of the views' own launches (the kernel variant that suits
-                                the rays of all of them) on four concurrent branches, largest views first */
+    MM_BATCH_GRAPH = 2       /* the views' own launches (the kernel variant that suits the rays of all of
+                                them) on up to 16 concurrent branches, largest views first */
 } mm_batch_schedule;
 
 typedef struct mm_batch_options {
@@ -441,12 +441,11 @@ int mm_batch_options_default(mm_batch_options* o);
 
 /* Renders n views (full frames, hardware sampler, fast math, plain or surrogate cone) with the shared textures:
  * blocks of all views in one grid (MM_BATCH_BLOCKS; one launch per 72 views), a persistent kernel
- * whose warps take tiles of all views from one queue (MM_BATCH_PERSISTENT), or one CUDA graph of the
- * views' own launches on concurrent branches (MM_BATCH_GRAPH, re-captured and updated in place on
- * every call).  The host-side records are
- * staged in pinned memory owned by the context; a call waits for the previous batch of the same
- * context to finish reading them.  The graph is re-captured when the view count or the options
- * change. */
+ * whose warps take tiles of all views from one queue (MM_BATCH_PERSISTENT), or the views' own launches
+ * on concurrent branches forked from `stream` and joined into it (MM_BATCH_GRAPH).  The first two
+ * replay a CUDA graph (use_graph; re-captured when the view count or the options change), and their
+ * host-side records are staged in pinned memory owned by the context: such a call waits for the
+ * previous one of the same context to finish reading them. */
 int mm_clouds_march_batch(mm_context ctx, const mm_view* views, int n, const mm_scene_textures* tex,
                           const mm_batch_options* opt, void* stream);
 

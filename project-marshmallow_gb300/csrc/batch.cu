@@ -5,10 +5,12 @@
 // each, tw x 32/tw pixels), numbered view after view; persistent warps take chunks of `grab`
 // consecutive tiles from one global counter, find the view by a binary search over the views'
 // first-tile indices, read that view's record from constant memory and march the tile's rays
-// exactly as march_tiled_kernel does; within a view the tile rows just above its horizon come first.  The record upload, the counter reset and the kernel are captured into
-// a CUDA graph once per (view count, options, textures) and replayed for later batches.  The
-// default schedule (MM_BATCH_BLOCKS) is one ordinary launch over 16x8-pixel blocks of all views
-// instead: blocks of one SM then cover compact neighbouring tiles, as in march_tiled_kernel.
+// exactly as march_tiled_kernel does; within a view the tile rows just above its horizon come first.
+// The record upload, the counter reset and the kernel are captured into a CUDA graph once per (view
+// count, options, textures) and replayed for later batches.  MM_BATCH_BLOCKS is one ordinary launch over
+// 16x8-pixel blocks of all views instead: blocks of one SM then cover compact neighbouring tiles, as in
+// march_tiled_kernel.  The default schedule (MM_BATCH_GRAPH) launches the views' own kernels on up to 16
+// concurrent branches.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -142,23 +144,32 @@ struct BatchState {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;  // the last batch that read the staging buffers
     int g_n = -1, g_tw = 0, g_grab = 0, g_grid = 0, g_launches = 0, g_sched = -1;
-    // MM_BATCH_GRAPH: capture streams (one per branch) and their fork/join events
-    static constexpr int kBranches = 4;
+    // MM_BATCH_GRAPH: one stream per branch and their fork/join events
+    static constexpr int kBranches = 16;
     cudaStream_t branch[kBranches] = {};
     cudaEvent_t fork = nullptr, join[kBranches] = {};
 };
 
-// Views in order of decreasing ray count, dealt round-robin to the graph's branches (the longest
-// launches start first on every branch; the small ones fill the others' tails).
-int capture_views(mm_context ctx, BatchState* b, const mm_view* views, int n, const mm_scene_textures* tex,
-                  const mm_batch_options& o, cudaGraph_t* out) {
+// MM_BATCH_GRAPH: the views' own launches, in order of decreasing ray count, dealt round-robin to the
+// branch streams (the longest launches start first on every branch; the small ones fill the others'
+// tails), between a fork from the caller's stream and a join into it.  The launches take their records
+// by value, so a call waits for nothing on the host and the next one is queued while it runs.
+// Capturing them into a graph, updating the executable one and waiting for the previous batch cost
+// ~60 us a view on the host with the GPU idle.  A view's kernel is chosen as if half the rays of the
+// others were its own: they share the GPU, but not for the whole of its time.  Six cube faces and three or six
+// smaller cameras, us on GB300, start (graph, 4 branches) -> launches on 4 / 8 / 16 branches with all of
+// the others' rays counted / on 16 with half: 512 + 1280..975 wide 2662 -> 2353 / 2306 / 2279 / 2273;
+// 200 + 520..398 741 -> 768 / 563 / 547 / 546; 128 + 400..278 727 -> 650 / 479 / 387 / 340; a 64x64 cube
+// and one camera 348 -> 144 / 86 / 86 / 86.
+int launch_views(mm_context ctx, BatchState* b, const mm_view* views, int n, const mm_scene_textures* tex,
+                 const mm_batch_options& o, cudaStream_t s) {
     constexpr int K = BatchState::kBranches;
     if (!b->fork) {
-        MM_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
         for (int k = 0; k < K; ++k) {
-            MM_CUDA_TRY(cudaStreamCreateWithFlags(&b->branch[k], cudaStreamNonBlocking));
-            MM_CUDA_TRY(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
+            if (!b->branch[k]) MM_CUDA_TRY(cudaStreamCreateWithFlags(&b->branch[k], cudaStreamNonBlocking));
+            if (!b->join[k]) MM_CUDA_TRY(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
         }
+        MM_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
     }
     int* order = new (std::nothrow) int[n];
     if (!order) return mm::fail(MM_ERR_OUT_OF_MEMORY, "batch: host allocation");
@@ -175,14 +186,11 @@ int capture_views(mm_context ctx, BatchState* b, const mm_view* views, int n, co
     }
     long long rays = 0;  // of all views: they run side by side
     for (int i = 0; i < n; ++i) rays += (long long)views[i].out.width * views[i].out.height;
+    const int used = o.surrogate ? 1 : (n < K ? n : K);
     int r = MM_OK;
-    cudaError_t e = cudaStreamBeginCapture(b->branch[0], cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) {
-        delete[] order;
-        return mm::cuda_fail(e, "batch graph capture");
-    }
-    cudaEventRecord(b->fork, b->branch[0]);
-    for (int k = 1; k < K; ++k) cudaStreamWaitEvent(b->branch[k], b->fork, 0);
+    cudaError_t e = cudaEventRecord(b->fork, s);
+    for (int k = 0; k < used && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(b->branch[k], b->fork, 0);
+    if (e != cudaSuccess) r = mm::cuda_fail(e, "batch fork");
     for (int i = 0; i < n && r == MM_OK; ++i) {
         const mm_view& v = views[order[i]];
         mm_march_options mo;
@@ -198,22 +206,16 @@ int capture_views(mm_context ctx, BatchState* b, const mm_view* views, int n, co
         else
             r = mm::launch_march_fast(p, MM_SAMPLER_HARDWARE, o.density_format, MM_SCHEDULE_TILED, 0, ctx->d_work,
                                       ctx->num_sms, b->branch[o.surrogate ? 0 : i % K],
-                                      o.surrogate ? 0 : rays - (long long)v.out.width * v.out.height);
+                                      o.surrogate ? 0 : (rays - (long long)v.out.width * v.out.height) / 2);
     }
-    for (int k = 1; k < K; ++k) {
-        cudaEventRecord(b->join[k], b->branch[k]);
-        cudaStreamWaitEvent(b->branch[0], b->join[k], 0);
-    }
-    cudaGraph_t g = nullptr;
-    e = cudaStreamEndCapture(b->branch[0], &g);
     delete[] order;
-    if (r == MM_OK && e != cudaSuccess) r = mm::cuda_fail(e, "batch graph capture");
-    if (r != MM_OK) {
-        if (g) cudaGraphDestroy(g);
-        return r;
+    // join in every case, so that the caller's stream never runs ahead of the views
+    for (int k = 0; k < used; ++k) {
+        e = cudaEventRecord(b->join[k], b->branch[k]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->join[k], 0);
+        if (e != cudaSuccess && r == MM_OK) r = mm::cuda_fail(e, "batch join");
     }
-    *out = g;
-    return MM_OK;
+    return r;
 }
 
 BatchState* state_of(mm_context ctx) { return reinterpret_cast<BatchState*>(ctx->batch); }
@@ -348,14 +350,8 @@ extern "C" int mm_clouds_march_batch(mm_context ctx, const mm_view* views, int n
         if (!ctx->batch) return fail(MM_ERR_OUT_OF_MEMORY, "batch: host allocation");
     }
     BatchState* b = state_of(ctx);
-    if (!b->done) MM_CUDA_TRY(cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming));
-    // The previous batch's upload reads the pinned staging buffers: let it finish first.
-    MM_CUDA_TRY(cudaEventSynchronize(b->done));
     if (o.schedule == MM_BATCH_GRAPH) {
-        // Each view's own launch (its kernel variant, uniforms by value) captured on the branches,
-        // then applied to the executable graph (cudaGraphExecUpdate) or instantiated anew.
-        cudaGraph_t g = nullptr;
-        if (o.surrogate) {  // the deferred-sample records of the largest view, allocated before the capture
+        if (o.surrogate) {  // the deferred-sample records of the largest view
             size_t most = 0;
             for (int i = 0; i < n; ++i) {
                 const size_t px = (size_t)views[i].out.width * views[i].out.height;
@@ -364,32 +360,11 @@ extern "C" int mm_clouds_march_batch(mm_context ctx, const mm_view* views, int n
             int rr = mm::surrogate_reserve(ctx, most);
             if (rr) return rr;
         }
-        int r = capture_views(ctx, b, views, n, tex, o, &g);
-        if (r) return r;
-        bool updated = false;
-        if (b->exec && b->g_sched == MM_BATCH_GRAPH && b->g_n == n) {
-            cudaGraphExecUpdateResultInfo info;
-            updated = cudaGraphExecUpdate(b->exec, g, &info) == cudaSuccess;
-            if (!updated) cudaGetLastError();  // clear the update failure; instantiate below
-        }
-        if (updated) {
-            cudaGraphDestroy(g);
-        } else {
-            drop_graph(b);
-            b->graph = g;
-            cudaError_t e = cudaGraphInstantiate(&b->exec, g, 0);
-            if (e != cudaSuccess) {
-                drop_graph(b);
-                return mm::cuda_fail(e, "batch graph instantiate");
-            }
-            b->g_n = n;
-            b->g_sched = MM_BATCH_GRAPH;
-        }
-        MM_CUDA_TRY(cudaGraphLaunch(b->exec, (cudaStream_t)stream));
-        mm::count_launch(n);
-        MM_CUDA_TRY(cudaEventRecord(b->done, (cudaStream_t)stream));
-        return MM_OK;
+        return launch_views(ctx, b, views, n, tex, o, (cudaStream_t)stream);
     }
+    if (!b->done) MM_CUDA_TRY(cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming));
+    // The previous batch's upload reads the pinned staging buffers: let it finish first.
+    MM_CUDA_TRY(cudaEventSynchronize(b->done));
     int r = ensure_capacity(b, n);
     if (r) return r;
     const int th = 32 / o.warp_tile_w;
