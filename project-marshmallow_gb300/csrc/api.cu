@@ -157,12 +157,40 @@ int make_texture(int w, int h, int d, int ch, mm_texture* out) {
     t->depth = d;
     t->channels = ch;
     cudaGetDevice(&t->device);
-    cudaError_t e = cudaMalloc(&t->texels, (size_t)w * h * d * ch);
+    // the erosion bound stands behind the texels
+    const size_t n = (size_t)w * h * d * ch, at = (n + 15) / 16 * 16;
+    cudaError_t e = cudaMalloc(&t->texels, at + sizeof(float));
     if (e != cudaSuccess) {
         delete t;
         return mm::cuda_fail(e, "texture texels");
     }
+    if (d > 1 && ch == 4) t->erosion_max = reinterpret_cast<const float*>(t->texels + at);
     *out = t;
+    return MM_OK;
+}
+
+// Largest erosion (0.625 r + 0.25 g + 0.125 b, compute-clouds.comp:224) of a texel: cloudHiRes can give
+// no sample more than this, which lets the march tell without a fetch that a thin sample is eroded away.
+// *out starts at zero bits; the values are not negative, so their bits order as they do.
+__global__ void __launch_bounds__(256) erosion_max_kernel(const uchar4* texels, size_t n, float* out) {
+    float m = 0.0f;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uchar4 c = texels[i];
+        m = fmaxf(m, 0.625f * c.x + 0.25f * c.y + 0.125f * c.z);
+    }
+    const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m * (1.0f / 255.0f)));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(out), bits);
+}
+
+int find_erosion_max(mm_texture t, cudaStream_t s) {
+    if (!t->erosion_max) return MM_OK;
+    float* out = const_cast<float*>(t->erosion_max);
+    const size_t n = (size_t)t->width * t->height * t->depth;
+    MM_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float), s));
+    erosion_max_kernel<<<(unsigned)(n < 256 * 1024 ? (n + 255) / 256 : 1024), 256, 0, s>>>(
+        reinterpret_cast<const uchar4*>(t->texels), n, out);
+    MM_CUDA_TRY(cudaGetLastError());
+    mm::count_launch();
     return MM_OK;
 }
 
@@ -255,7 +283,8 @@ int mm_noise_generate(const mm_noise_desc* desc, mm_texture* out, void* stream) 
     mm_texture t = nullptr;
     if ((r = make_texture(w, h, d, ch, &t))) return r;
     cudaStream_t s = (cudaStream_t)stream;
-    if ((r = mm_noise_fill(desc, t->texels, (size_t)w * h * d * ch, stream)) || (r = build_hw_copy(t, MM_FORMAT_UNORM8, s))) {
+    if ((r = mm_noise_fill(desc, t->texels, (size_t)w * h * d * ch, stream)) || (r = find_erosion_max(t, s)) ||
+        (r = build_hw_copy(t, MM_FORMAT_UNORM8, s))) {
         cudaStreamSynchronize(s);
         release(t);
         return r;
@@ -281,7 +310,7 @@ int mm_texture_create(const void* texels, int src_is_device, int width, int heig
         release(t);
         return mm::cuda_fail(e, "texture upload");
     }
-    if ((r = build_hw_copy(t, format, s))) {
+    if ((r = find_erosion_max(t, s)) || (r = build_hw_copy(t, format, s))) {
         cudaStreamSynchronize(s);
         release(t);
         return r;
@@ -549,6 +578,7 @@ void mm::fill_march_launch(const mm_uniforms& u, const mm_scene_textures* tex, c
     p.uv_h = o.ref_uv_1080p ? 1080.0f : (float)out.height;
     p.coverage_offset = o.coverage_offset;
     p.counters = reinterpret_cast<unsigned long long*>(o.d_counters);
+    p.erosion_max = p.counters ? nullptr : tex->hi_res->erosion_max;  // a counting launch runs every sample
     march_host_consts(p);
 }
 

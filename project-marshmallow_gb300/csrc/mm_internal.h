@@ -39,6 +39,7 @@ struct mm_texture_s {
     int width = 0, height = 0, depth = 0, channels = 0;
     int format = MM_FORMAT_UNORM8;   // format of the hardware-filtered copy
     uint8_t* texels = nullptr;       // device, width*height*depth*channels bytes
+    const float* erosion_max = nullptr;  // device, 3D RGBA only: largest 0.625 r + 0.25 g + 0.125 b of a texel
     cudaArray_t array = nullptr;
     cudaTextureObject_t tex = 0;
     int device = 0;
@@ -90,6 +91,7 @@ struct MarchLaunch {
     float uv_w, uv_h;
     float coverage_offset;
     unsigned long long* counters;
+    const float* erosion_max;  // of the hi-res texture; null: every sample with density takes its cloudHiRes
     int row_split;  // tiled march: block rows [0, row_split) run in reverse order first (0 = launch order)
     // Per-frame constants of the production-arithmetic march, computed once on the host
     // (march_host_consts) so the kernels read them from the parameter bank instead of holding them
