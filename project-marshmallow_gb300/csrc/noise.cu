@@ -51,10 +51,8 @@ __device__ __forceinline__ uint32_t stream_seed(uint32_t seed, int kind, int ch,
     return hash32(seed ^ hash32(0x9E3779B9u * (uint32_t)(1 + kind * 64 + ch * 8 + oct)));
 }
 
-__device__ __forceinline__ int wrapi(int c, int f) {
-    int m = c % f;
-    return m < 0 ? m + f : m;
-}
+// c modulo f; every frequency of the generators is a power of two
+__device__ __forceinline__ int wrapi(int c, int f) { return c & (f - 1); }
 
 __device__ __forceinline__ float lattice(int i, int n, int f) {
     return __fdiv_rn((float)((2 * i + 1) * f), (float)(2 * n));
@@ -89,15 +87,6 @@ __device__ float worley3(float qx, float qy, float qz, int f, uint32_t s) {
         }
     }
     return 1.0f - fminf(__fsqrt_rn(best), 1.0f);
-}
-
-__device__ float worley_fbm(int i, int j, int k, int n, int f, uint32_t seed, int kind, int ch) {
-    const float a = worley3(lattice(i, n, f), lattice(j, n, f), lattice(k, n, f), f, stream_seed(seed, kind, ch, 0));
-    const float b = worley3(lattice(i, n, 2 * f), lattice(j, n, 2 * f), lattice(k, n, 2 * f), 2 * f,
-                            stream_seed(seed, kind, ch, 1));
-    const float c = worley3(lattice(i, n, 4 * f), lattice(j, n, 4 * f), lattice(k, n, 4 * f), 4 * f,
-                            stream_seed(seed, kind, ch, 2));
-    return (0.625f * a + 0.25f * b) + 0.125f * c;
 }
 
 __device__ __forceinline__ float fade(float t) { return t * t * t * (t * (t * 6.0f - 15.0f) + 10.0f); }
@@ -180,39 +169,240 @@ __device__ float value2(float qx, float qy, int f, uint32_t s) {
     return lerpf(lerpf(v00, v10, u), lerpf(v01, v11, u), v);
 }
 
-// 3D density volumes: a block is a 32x8 (x,y) tile of one z slice; each thread one texel, one
-// 4-byte store, so a warp writes 128 contiguous bytes.
-__global__ void __launch_bounds__(256) volume_kernel(int kind, uint32_t seed, int n, uchar4* out) {
-    const int i = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 8 + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= n || j >= n) return;
-    uchar4 t;
-    if (kind == MM_NOISE_LOWRES_PERLIN_WORLEY) {
-        const int f = 4;
-        float sum = 0.0f, amp = 1.0f, norm = 0.0f;
+// ---------------------------------------------------------------- 3D density volumes
+//
+// A block makes a tile of 32 x 2 x kRun texels (x, y, z).  Its work is split into units of two warps (one
+// lane a column of kRun texels): one unit per Worley channel and, for the low-res volume, one for the
+// Perlin octaves.  For each octave a unit first hashes the cells its tile can reach into shared memory,
+// once per cell instead of 27 times per texel, then every lane takes its 27 neighbours from there.  The
+// texels of a column that lie in the same cell along z (4 at a time, 2, or 1: the same for every lane) go
+// through a neighbour together: its x and y distances are theirs in common, which leaves a subtraction,
+// a product, a sum and a minimum each.  Every float operation is worley3's own, so the texels are the same
+// bytes.  Where an octave has more cells in reach than the table holds (more than about half a cell per
+// texel), its texels are computed one by one as before.
+// Bound by FP32 issue: 27 distances x 12 octaves a texel.  us at the start -> with the tables -> with packed FP32
+// operations: low-res 128^3 1229 -> 226 -> 201, 64^3 164 -> 56 -> 52; hi-res 32^3 27 -> 11, 64^3 109 -> 27 -> 25.
+// (Passing over rows of cells no closer than the distance found so far costs what it saves: 232 -> 240.)
+constexpr int kCells = 680;         // table entries of a Worley unit: 32 x 2 x 8 texels at 0.55 cells a texel
+constexpr int kPerlinCells = 256;   // of the Perlin unit, whose octaves are the coarse ones
+
+// Two floats in one register pair; the packed operations round each half as the scalar ones do.
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// The square, rounded by itself: a packed product followed by a packed sum is contracted by the assembler
+// even at -fmad=false, a product already fused with + 0 is not.
+__device__ __forceinline__ unsigned long long square2(unsigned long long a) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(r) : "l"(a), "l"(0ull));
+    return r;
+}
+
+// Minimum squared distance (at most 1) to the 27 neighbours for M texels that share their cell; the
+// texels' fractions are (fx, fy, fz[m]) and `at` is the table entry of neighbour (-1, -1, -1).  The
+// distances along x and y, and those of two texels along z, go through packed FP32 operations.
+template <int M>
+__device__ __forceinline__ void nearest(const float* at, int cells, int nx, int nxy, float fx, float fy, const float* fz,
+                                        float* best) {
+    unsigned long long nz[M / 2 + 1];
+#pragma unroll
+    for (int m = 0; m < M; ++m) best[m] = 1.0f;
+#pragma unroll
+    for (int m = 0; m + 1 < M; m += 2) nz[m / 2] = pair(-fz[m], -fz[m + 1]);
+    const unsigned long long nfxy = pair(-fx, -fy);
 #pragma unroll 1
-        for (int o = 0; o < 3; ++o) {
-            const int fo = f << o;
-            sum += amp * perlin3(lattice(i, n, fo), lattice(j, n, fo), lattice(k, n, fo), fo,
-                                 stream_seed(seed, kind, 0, 4 + o));
+    for (int dz = 0; dz < 3; ++dz) {
+        const float oz = (float)(dz - 1);
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+            const float* row = at + dy * nx;
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                unsigned long long e = add2(pair(row[dx], row[cells + dx]), pair((float)(dx - 1), (float)(dy - 1)));
+                e = add2(e, nfxy);
+                e = square2(e);
+                float ex, ey;
+                unpair(e, ex, ey);
+                const float exy = ex + ey;
+                const float pz = oz + row[2 * cells + dx];
+                if (M == 1) {
+                    const float ez = pz - fz[0];
+                    best[0] = fminf(best[0], exy + ez * ez);
+                } else {
+                    const unsigned long long pz2 = pair(pz, pz), exy2 = pair(exy, exy);
+#pragma unroll
+                    for (int m = 0; m + 1 < M; m += 2) {
+                        unsigned long long ez = add2(pz2, nz[m / 2]);
+                        ez = add2(exy2, square2(ez));
+                        float d0, d1;
+                        unpair(ez, d0, d1);
+                        best[m] = fminf(best[m], d0);
+                        best[m + 1] = fminf(best[m + 1], d1);
+                    }
+                }
+            }
+        }
+        at += nxy;
+    }
+}
+
+// Barrier of a unit's two warps: units take their octaves at their own pace.
+__device__ __forceinline__ void unit_sync(int unit) { asm volatile("bar.sync %0, 64;" ::"r"(unit + 1) : "memory"); }
+
+template <int kRun>
+__global__ void __launch_bounds__(320) volume_kernel(int kind, uint32_t seed, int n, uchar4* out) {
+    constexpr unsigned full = 0xffffffffu;
+    __shared__ float s_table[4 * 3 * kCells + 3 * kPerlinCells];
+    __shared__ float s_sum[kRun][320];  // each thread's own octave sums, and the Perlin unit's for unit 0
+    __shared__ __align__(4) uint8_t s_out[kRun][64][4];
+    const bool low = kind == MM_NOISE_LOWRES_PERLIN_WORLEY;
+    const int worleys = low ? 4 : 3;
+    const int unit = threadIdx.x >> 6, t = threadIdx.x & 63, lane = t & 31;
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 2, k0 = blockIdx.z * kRun;
+    const int i = min(i0 + lane, n - 1);  // columns outside: a neighbour's
+    const bool perlin = unit == worleys;
+    const int cap = perlin ? kPerlinCells : kCells;
+    float* const table = s_table + unit * 3 * kCells;
+    // first octave of the unit's channel: low-res R (and the Perlin octaves) 4, G/B/A 4/8/16; hi-res 2/4/8
+    const int f0 = low ? (unit == 0 || perlin ? 4 : 4 << (unit - 1)) : 2 << unit;
+    float amp = 1.0f, norm = 0.0f;
+#pragma unroll 1
+    for (int o = 0; o < 3; ++o) {
+        const int f = f0 << o;
+        const uint32_t s = stream_seed(seed, kind, perlin ? 0 : unit, perlin ? 4 + o : o);
+        // lattice points: this lane's x, the tile's two y and (lane r) its z
+        const float qx = lattice(i, n, f), qy0 = lattice(j0, n, f), qy1 = lattice(min(j0 + 1, n - 1), n, f);
+        const float ql = lattice(min(k0 + min(lane, kRun - 1), n - 1), n, f);
+        const float qy = t < 32 ? qy0 : qy1;
+        const float fx = qx - floorf(qx), fy = qy - floorf(qy), fl = ql - floorf(ql);
+        const int cx = (int)floorf(qx), cy = (int)floorf(qy), cl = (int)floorf(ql);
+        // cells in reach of the tile: x0 .. x0 + nx - 1 and so on
+        const int x0 = __shfl_sync(full, cx, 0) - 1, nx = __shfl_sync(full, cx, 31) - x0 + 2;
+        const int y0 = (int)floorf(qy0) - 1, ny = (int)floorf(qy1) - y0 + 2;
+        const int z0 = __shfl_sync(full, cl, 0) - 1, nz = __shfl_sync(full, cl, 31) - z0 + 2;
+        const int nxy = nx * ny, cells = nxy * nz;
+        const bool tabled = cells <= cap;
+        if (o) unit_sync(unit);  // the last octave's entries are read
+        if (tabled) {
+            // c / nxy and q / nx by multiplication: exact for entries below 2^16
+            const uint32_t by_xy = 0xffffffffu / (uint32_t)nxy + 1u, by_x = 0xffffffffu / (uint32_t)nx + 1u;
+            for (int c = t; c < cells; c += 64) {
+                const int z = (int)__umulhi((uint32_t)c, by_xy), q = c - z * nxy;
+                const int y = (int)__umulhi((uint32_t)q, by_x), x = q - y * nx;
+                const uint32_t h = hash3(wrapi(x0 + x, f), wrapi(y0 + y, f), wrapi(z0 + z, f), s);
+                if (perlin) {  // the gradient of lattice point (x, y, z)
+                    table[c] = grad3(h, 1.0f, 0.0f, 0.0f);
+                    table[cap + c] = grad3(h, 0.0f, 1.0f, 0.0f);
+                    table[2 * cap + c] = grad3(h, 0.0f, 0.0f, 1.0f);
+                } else {  // the feature point of cell (x, y, z)
+                    table[c] = rand01(h);
+                    table[cap + c] = rand01(hash32(h + 0x9E3779B9u));
+                    table[2 * cap + c] = rand01(hash32(h + 0x3C6EF372u));
+                }
+            }
+        }
+        unit_sync(unit);
+        const float* const column = table + (cy - 1 - y0) * nx + (cx - 1 - x0);  // neighbour (-1, -1), plane z0
+        const float weight = o == 0 ? 0.625f : (o == 1 ? 0.25f : 0.125f);
+        if (perlin) {
+            const float u = fade(fx), v = fade(fy);
+#pragma unroll 1
+            for (int r = 0; r < kRun; ++r) {
+                const float fz = __shfl_sync(full, fl, r);
+                float p;
+                if (tabled) {
+                    const float* at = column + (__shfl_sync(full, cl, r) - z0) * nxy + nx + 1;
+                    float g[8];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const float* e = at + (c & 1) + (c & 2 ? nx : 0) + (c & 4 ? nxy : 0);
+                        const float x = c & 1 ? fx - 1.0f : fx, y = c & 2 ? fy - 1.0f : fy, z = c & 4 ? fz - 1.0f : fz;
+                        g[c] = (e[0] * x + e[kPerlinCells] * y) + e[2 * kPerlinCells] * z;
+                    }
+                    const float w = fade(fz);
+                    p = lerpf(lerpf(lerpf(g[0], g[1], u), lerpf(g[2], g[3], u), v),
+                              lerpf(lerpf(g[4], g[5], u), lerpf(g[6], g[7], u), v), w);
+                } else {
+                    p = perlin3(qx, qy, __shfl_sync(full, ql, r), f, s);
+                }
+                s_sum[r][threadIdx.x] = (o ? s_sum[r][threadIdx.x] : 0.0f) + amp * p;
+            }
             norm += amp;
             amp *= 0.5f;
+        } else if (tabled) {
+            auto add = [&](int r, float best) {
+                const float w = weight * (1.0f - fminf(__fsqrt_rn(best), 1.0f));
+                s_sum[r][threadIdx.x] = o ? s_sum[r][threadIdx.x] + w : w;
+            };
+#pragma unroll 1
+            for (int r = 0; r < kRun;) {  // the next 4, 2 or 1 texels of the column that share a cell
+                const int c = __shfl_sync(full, cl, r);
+                const bool two = r + 1 < kRun && __shfl_sync(full, cl, r + 1) == c;
+                const bool four = r + 3 < kRun && __shfl_sync(full, cl, r + 3) == c;
+                const float* at = column + (c - 1 - z0) * nxy;
+                float fz[4], best[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) fz[m] = __shfl_sync(full, fl, r + m);
+                if (four) {
+                    nearest<4>(at, kCells, nx, nxy, fx, fy, fz, best);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) add(r + m, best[m]);
+                    r += 4;
+                } else if (two) {
+                    nearest<2>(at, kCells, nx, nxy, fx, fy, fz, best);
+                    add(r, best[0]);
+                    add(r + 1, best[1]);
+                    r += 2;
+                } else {
+                    nearest<1>(at, kCells, nx, nxy, fx, fy, fz, best);
+                    add(r, best[0]);
+                    r += 1;
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int r = 0; r < kRun; ++r) {
+                const float w = weight * worley3(qx, qy, __shfl_sync(full, ql, r), f, s);
+                s_sum[r][threadIdx.x] = o ? s_sum[r][threadIdx.x] + w : w;
+            }
         }
-        const float p01 = __fdiv_rn(sum, norm) * 0.5f + 0.5f;
-        const float wf = worley_fbm(i, j, k, n, f, seed, kind, 0);
-        const float pw = __fdiv_rn(p01 - (wf - 1.0f), 1.0f - (wf - 1.0f));
-        t.x = quantize(1.64f * pw + -0.593f);
-        t.y = quantize(0.866f * worley_fbm(i, j, k, n, 4, seed, kind, 1) + 0.271f);
-        t.z = quantize(0.866f * worley_fbm(i, j, k, n, 8, seed, kind, 2) + 0.271f);
-        t.w = quantize(0.866f * worley_fbm(i, j, k, n, 16, seed, kind, 3) + 0.271f);
-    } else {
-        t.x = quantize(0.866f * worley_fbm(i, j, k, n, 2, seed, kind, 0) + 0.271f);
-        t.y = quantize(0.866f * worley_fbm(i, j, k, n, 4, seed, kind, 1) + 0.271f);
-        t.z = quantize(0.866f * worley_fbm(i, j, k, n, 8, seed, kind, 2) + 0.271f);
-        t.w = 0;
     }
-    out[((size_t)k * n + j) * n + i] = t;
+    // ---- texels: R of the low-res volume needs the Perlin unit's sums
+    if (perlin) {
+#pragma unroll 1
+        for (int r = 0; r < kRun; ++r)
+            s_sum[r][threadIdx.x] = __fdiv_rn(s_sum[r][threadIdx.x], norm) * 0.5f + 0.5f;
+    }
+    __syncthreads();
+    if (!perlin) {
+#pragma unroll 1
+        for (int r = 0; r < kRun; ++r) {
+            const float wf = s_sum[r][threadIdx.x];
+            if (low && unit == 0) {
+                const float pw = __fdiv_rn(s_sum[r][4 * 64 + t] - (wf - 1.0f), 1.0f - (wf - 1.0f));
+                s_out[r][t][0] = quantize(1.64f * pw + -0.593f);
+            } else {
+                s_out[r][t][unit] = quantize(0.866f * wf + 0.271f);
+            }
+            if (!low && unit == 0) s_out[r][t][3] = 0;
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kRun * 64; e += blockDim.x) {
+        const int x = i0 + (e & 31), y = j0 + ((e >> 5) & 1), z = k0 + (e >> 6);
+        if (x < n && y < n && z < n)
+            out[((size_t)z * n + y) * n + x] = *reinterpret_cast<const uchar4*>(s_out[e >> 6][e & 63]);
+    }
 }
 
 __device__ float curl_potential(float qx, float qy, uint32_t seed) {
@@ -227,16 +417,26 @@ __device__ float curl_potential(float qx, float qy, uint32_t seed) {
     return __fdiv_rn(sum, norm);
 }
 
+// Four lanes a texel, one potential each: 128^2 texels are too few to fill the GPU with one thread each
+// (12.5 -> 6.4 us).
 __global__ void __launch_bounds__(256) curl_kernel(uint32_t seed, int w, int h, uchar2* out) {
-    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int part = threadIdx.x & 3;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 2);
     const int j = blockIdx.y * 8 + threadIdx.y;
-    if (i >= w || j >= h) return;
-    const float xm = __fdiv_rn((float)(4 * i + 1), (float)(4 * w)), xp = __fdiv_rn((float)(4 * i + 3), (float)(4 * w));
-    const float ym = __fdiv_rn((float)(4 * j + 1), (float)(4 * h)), yp = __fdiv_rn((float)(4 * j + 3), (float)(4 * h));
-    const float xc = __fdiv_rn((float)(2 * i + 1), (float)(2 * w)), yc = __fdiv_rn((float)(2 * j + 1), (float)(2 * h));
-    const float dpx = (curl_potential(xp, yc, seed) - curl_potential(xm, yc, seed)) * (float)(2 * w);
-    const float dpy = (curl_potential(xc, yp, seed) - curl_potential(xc, ym, seed)) * (float)(2 * h);
-    out[(size_t)j * w + i] = make_uchar2(quantize(0.5f + 0.03f * dpy), quantize(0.5f - 0.03f * dpx));
+    const int ic = min(i, w - 1), jc = min(j, h - 1);
+    // x + a quarter texel, x - a quarter, y + a quarter, y - a quarter
+    const float x = part == 0   ? __fdiv_rn((float)(4 * ic + 3), (float)(4 * w))
+                    : part == 1 ? __fdiv_rn((float)(4 * ic + 1), (float)(4 * w))
+                                : __fdiv_rn((float)(2 * ic + 1), (float)(2 * w));
+    const float y = part == 2   ? __fdiv_rn((float)(4 * jc + 3), (float)(4 * h))
+                    : part == 3 ? __fdiv_rn((float)(4 * jc + 1), (float)(4 * h))
+                                : __fdiv_rn((float)(2 * jc + 1), (float)(2 * h));
+    const float p = curl_potential(x, y, seed);
+    const float other = __shfl_xor_sync(0xffffffffu, p, 1);
+    const float d = (p - other) * (float)(part == 0 ? 2 * w : 2 * h);  // lanes 0 and 2: dp/dx, dp/dy
+    const float dpy = __shfl_down_sync(0xffffffffu, d, 2);
+    if (part == 0 && i < w && j < h)
+        out[(size_t)j * w + i] = make_uchar2(quantize(0.5f + 0.03f * dpy), quantize(0.5f - 0.03f * d));
 }
 
 __global__ void __launch_bounds__(256) weather_kernel(uint32_t seed, int w, int h, uchar4* out) {
@@ -430,13 +630,24 @@ int launch_noise(int kind, uint32_t seed, int w, int h, int d, uint8_t* out, cud
     switch (kind) {
         case MM_NOISE_LOWRES_PERLIN_WORLEY:
         case MM_NOISE_HIRES_WORLEY: {
-            dim3 grid((w + 31) / 32, (h + 7) / 8, d);
-            volume_kernel<<<grid, dim3(32, 8), 0, s>>>(kind, seed, w, reinterpret_cast<uchar4*>(out));
+            const int threads = kind == MM_NOISE_LOWRES_PERLIN_WORLEY ? 320 : 192;
+            uchar4* texels = reinterpret_cast<uchar4*>(out);
+            // Texels of a column: longer columns hash fewer cells a texel, shorter ones make more blocks.
+            // 8 / 4 / 2 / 1 texels, us: low-res 128^3 224 / 261 / 388 / -, 64^3 64 / 58 / 62 / -, 40^3 - / 35 /
+            // 39 / 47, 24^3 - / 23 / 15 / 15; hi-res 64^3 27 / 29 / 37 / -, 48^3 - / 21 / 27 / 37, 32^3 - / 17 /
+            // 11 / 13, 16^3 - / 18 / 13 / 9.
+            const int run = w >= 64 ? 8 : (w >= 40 ? 4 : (w >= 28 ? 2 : 1));
+            const dim3 grid((w + 31) / 32, (h + 1) / 2, (d + run - 1) / run);
+            switch (run) {
+                case 8: volume_kernel<8><<<grid, threads, 0, s>>>(kind, seed, w, texels); break;
+                case 4: volume_kernel<4><<<grid, threads, 0, s>>>(kind, seed, w, texels); break;
+                case 2: volume_kernel<2><<<grid, threads, 0, s>>>(kind, seed, w, texels); break;
+                default: volume_kernel<1><<<grid, threads, 0, s>>>(kind, seed, w, texels); break;
+            }
             break;
         }
         case MM_NOISE_CURL2D:
-            curl_kernel<<<dim3((w + 31) / 32, (h + 7) / 8), dim3(32, 8), 0, s>>>(seed, w, h,
-                                                                                 reinterpret_cast<uchar2*>(out));
+            curl_kernel<<<dim3((w + 7) / 8, (h + 7) / 8), dim3(32, 8), 0, s>>>(seed, w, h, reinterpret_cast<uchar2*>(out));
             break;
         case MM_NOISE_WEATHER:
             weather_kernel<<<dim3((w + 31) / 32, (h + 7) / 8), dim3(32, 8), 0, s>>>(seed, w, h,
