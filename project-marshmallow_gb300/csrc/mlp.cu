@@ -7,8 +7,8 @@
 //   z2 = h1 W2b^T + b2,       h2 = bf16(relu(z2))
 //   z3 = h2 W3b^T + b3,       h3 = relu(z3)              (FP32)
 //   y  = sigmoid(h3 . w4 + b4)                         (FP32, CUDA cores)
-// GEMMs accumulate in FP32 in tensor memory.  One CTA of 4 warps handles 128 samples at a time,
-// one sample per thread (= one TMEM lane) in the epilogues.
+// GEMMs accumulate in FP32 in tensor memory.  A CTA handles 128 samples at a time, one sample per TMEM
+// lane in the epilogues (inference: 4 warps, one thread a sample; training: 8 warps, two).
 //
 // Training (one kernel per step, then Adam): the backward pass keeps every GEMM on the tensor
 // cores.  With dz = 2 (y - t) y (1 - y) / B:
@@ -20,7 +20,7 @@
 // Weight-gradient GEMMs reduce over the 128 samples (K = 128) with M padded from 64 to 128 rows;
 // the ones row appended to B yields the bias gradient as one more output column.  Each layer's
 // weight gradient accumulates in its own tensor-memory columns over all the tiles a CTA trains on,
-// and the CTA adds it to a global FP32 buffer with atomics once, at its end.
+// and the CTA writes it as one row of partial sums at its end.
 //
 // The file also holds the tensor-core GEMM self-check used to validate the operand layout and the
 // MMA/TMEM protocol of tc.cuh on the device.
@@ -343,28 +343,58 @@ __global__ void __launch_bounds__(128, 5) infer_kernel(const __nv_bfloat16* __re
 //
 // Shared-memory tiles, all in the K-major layout of tc.cuh, each also read MN-major (transposed in
 // place) by the weight-gradient GEMMs:
-//   x  [128][32]:  features in columns 0..15, a ones column 16, zeros 17..31
+//   x  [128][32]:  features in columns 0..15, a ones column 16, zeros 17..31 (two, in turn)
 //   h1 [128][80], h2 [128][80]: activations in 0..63, ones column 64, zeros 65..79
-//   d  [128][128]: the delta of the current layer in 0..63, zeros 64..127
+//   d  [128][64]: a layer's delta (two, in turn).  As the weight-gradient GEMMs' A operand it is read with
+//                 M = 128: rows 64..127 come from whatever lies 1 KB further on and go to TMEM lanes that
+//                 nothing reads.
 // GEMMs per tile (D in TMEM, A x B^T):
 //   forward       z1 = x W1^T      A = x (K-major, K = 16)    B = W1 (K-major)
 //                 z2 = h1 W2^T, z3 = h2 W3^T
+//   deltas        d2 = (d3 W3) * [z2 > 0]  A = d (K-major, K = 64), B = W3 (MN-major: [out][in] read as [in][out])
+//                 d1 = (d2 W2) * [z1 > 0]
 //   weight grads  dW3|db3 += d3^T [h2 1]   A = d (MN-major, M = 128 rows of which 64 real, K = 128 samples)
 //                                          B = h2 (MN-major, N = 80)
 //                 dW2|db2 += d2^T [h1 1],  dW1|db1 += d1^T [x 1] (N = 32)
-//   deltas        d2 = (d3 W3) * [z2 > 0]  A = d (K-major, K = 64), B = W3 (MN-major: [out][in] read as [in][out])
-//                 d1 = (d2 W2) * [z1 > 0]
 // The ones columns turn the bias gradients into one more output column of the weight-gradient GEMMs.
+//
+// A tile is a chain of five GEMMs, each waited for and followed by an epilogue; the tensor cores are idle
+// most of the time and the chain's latency bounds the kernel.  Two warps share each 32 lanes of TMEM, one
+// for columns 0..31 and one for 32..63, so an epilogue is half as long; the weight-gradient GEMMs are issued
+// behind the delta GEMM of their phase and run during its epilogue (a later phase's wait covers them before
+// their operands are overwritten: the one issuing thread's MMAs complete in order); one barrier a phase.
+// One Adam step at batch 131,072, this kernel: 48.4 us with 128 threads a CTA, a weight-gradient GEMM on the
+// chain and six waits of two barriers -> 28.1 us (both under ncu).  The hidden layers' gradients keep every bit.
 
 struct TrainSmem {
-    SmemWeights w;
-    alignas(128) uint8_t x[128 * 32 * 2];
+    alignas(128) uint8_t x[2][128 * 32 * 2];
     alignas(128) uint8_t h1[128 * 80 * 2];
     alignas(128) uint8_t h2[128 * 80 * 2];
-    alignas(128) uint8_t d[128 * 128 * 2];
+    alignas(128) uint8_t d[2][128 * kHid * 2];
+    SmemWeights w;                // behind d: the read past its last rows stays inside
+    float out[4][kHid + 2];       // per 32 rows: gradients of w4 and b4, squared error
     uint64_t bar;
     uint32_t tslot;
 };
+static_assert(sizeof(SmemWeights) >= 1024, "operand reads 1 KB past d");
+
+// Floats of a CTA's row of partial gradients: the parameters, the squared error, rounded to 16 bytes.
+constexpr int kRow = (kParams + 1 + 3) / 4 * 4;
+
+// Sums v[0..31] over the warp's lanes; lane l gets the sum of v[l].  31 shuffles.
+__device__ __forceinline__ float warp_sum32(float* v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+        const bool upper = lane & half;
+#pragma unroll
+        for (int j = 0; j < half; ++j) {
+            const float keep = upper ? v[j + half] : v[j], give = upper ? v[j] : v[j + half];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+        }
+    }
+    return v[0];
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -373,18 +403,17 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // Writes a weight-gradient tile (TMEM columns [0, n_in] of lanes 0..63 from t_row, the last one the
-// bias) into the CTA's row of partial gradients.  Run by warps 0 and 1.
-__device__ __forceinline__ void flush_dw(uint32_t t_row, int o, int n_in, float* Gp, int off_w, int off_b) {
+// bias) into the CTA's row of partial gradients, columns [c0, c1).
+__device__ __forceinline__ void flush_dw(uint32_t t_row, int o, int n_in, int c0, int c1, float* Gp, int off_w, int off_b) {
     float v[16];
-    for (int c = 0; c < n_in + 16; c += 16) {
+    for (int c = c0; c < c1; c += 16) {
         tc::tmem_ld16(t_row + c, v);
+        if (c < n_in) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int i = c + j;
-            if (i < n_in)
-                Gp[off_w + o * n_in + i] = v[j];
-            else if (i == n_in)
-                Gp[off_b + o] = v[j];
+            for (int j = 0; j < 16; j += 4)
+                *reinterpret_cast<float4*>(Gp + off_w + o * n_in + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        } else {
+            Gp[off_b + o] = v[0];
         }
     }
 }
@@ -403,93 +432,91 @@ __device__ __forceinline__ void gemm_kk(uint32_t d_tmem, uint32_t sa, int a_cols
 // (cols / 8) * 128 bytes apart (descriptor leading-byte-offset field), MN groups 128 bytes.
 __device__ __forceinline__ void gemm_dw(uint32_t d_tmem, uint32_t s_d, uint32_t s_act, int n_cols, uint32_t accumulate) {
     const uint32_t idesc = tc::idesc_bf16_mn(128, n_cols, true, true);
-    const uint32_t ka = (128 / 8) * 128, kb = (uint32_t)(n_cols / 8) * 128;
+    const uint32_t ka = (kHid / 8) * 128, kb = (uint32_t)(n_cols / 8) * 128;
     for (int kk = 0; kk < 128 / 16; ++kk)
         tc::mma_bf16(d_tmem, tc::smem_desc(s_d + kk * 2 * ka, ka, 128), tc::smem_desc(s_act + kk * 2 * kb, kb, 128), idesc,
                      kk > 0 ? 1u : accumulate);
 }
 
-// Delta GEMM: D = d (K-major, K = 64, tile width 128) x W (the [64 out][64 in] forward weight tile
-// read MN-major as [in][out]).
+// Delta GEMM: D = d (K-major, K = 64) x W (the [64 out][64 in] forward weight tile read MN-major as
+// [in][out]).
 __device__ __forceinline__ void gemm_delta(uint32_t d_tmem, uint32_t s_d, uint32_t s_w) {
     const uint32_t idesc = tc::idesc_bf16_mn(128, kHid, false, true);
     const uint32_t kb = (kHid / 8) * 128;
     for (int kk = 0; kk < kHid / 16; ++kk)
-        tc::mma_bf16(d_tmem, tc::smem_desc(s_d + kk * 256, 128, (128 / 8) * 128),
-                     tc::smem_desc(s_w + kk * 2 * kb, kb, 128), idesc, kk > 0 ? 1u : 0u);
+        tc::mma_bf16(d_tmem, tc::smem_desc(s_d + kk * 256, 128, kb), tc::smem_desc(s_w + kk * 2 * kb, kb, 128), idesc,
+                     kk > 0 ? 1u : 0u);
 }
 
-// Features of the thread's row (zeros past n) and its target.
+// Half of the features of a row (zeros past n) and its target.
 __device__ __forceinline__ void load_sample(const __nv_bfloat16* __restrict__ X, const float* __restrict__ T, int row,
-                                            int n, uint4& a, uint4& b, float& t) {
+                                            int n, int half, uint4& a, float& t) {
     a = make_uint4(0, 0, 0, 0);
-    b = a;
     t = 0.0f;
     if (row < n) {
-        const uint4* src = reinterpret_cast<const uint4*>(X + (size_t)row * kIn);
-        a = __ldg(src);
-        b = __ldg(src + 1);
+        a = __ldg(reinterpret_cast<const uint4*>(X + (size_t)row * kIn) + half);
         t = __ldg(T + row);
     }
 }
 
-// Hidden-layer epilogue into an activation tile of width 80: + bias, ReLU, bf16.
-__device__ __forceinline__ void train_epilogue_hidden(uint32_t t_row, const float* bias, uint8_t* s, int r) {
+// Hidden-layer epilogue of columns c0 .. c0 + 31 into an activation tile of width 80: + bias, ReLU, bf16.
+__device__ __forceinline__ void train_epilogue_hidden(uint32_t t_row, const float* bias, uint8_t* s, int r, int c0) {
+    float v[32];
+    tc::tmem_ld32(t_row + c0, v);
 #pragma unroll
-    for (int c = 0; c < kHid; c += 16) {
-        float v[16];
-        tc::tmem_ld16(t_row + c, v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + bias[c + j], 0.0f);
-        *reinterpret_cast<uint4*>(s + tc::kmajor_offset(r, c, 80)) = tc::pack8_bf16(v);
-        *reinterpret_cast<uint4*>(s + tc::kmajor_offset(r, c + 8, 80)) = tc::pack8_bf16(v + 8);
+    for (int j = 0; j < 32; j += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + c0 + j);
+        v[j] = fmaxf(v[j] + b.x, 0.0f);
+        v[j + 1] = fmaxf(v[j + 1] + b.y, 0.0f);
+        v[j + 2] = fmaxf(v[j + 2] + b.z, 0.0f);
+        v[j + 3] = fmaxf(v[j + 3] + b.w, 0.0f);
     }
+#pragma unroll
+    for (int j = 0; j < 32; j += 8)
+        *reinterpret_cast<uint4*>(s + tc::kmajor_offset(r, c0 + j, 80)) = tc::pack8_bf16(v + j);
 }
 
-// Delta epilogue: (TMEM row) * [activation of the layer below > 0] as bf16 into d.
-__device__ __forceinline__ void train_epilogue_delta(uint32_t t_row, const uint8_t* act, uint8_t* d, int r) {
+// Delta epilogue of columns c0 .. c0 + 31: (TMEM row) * [activation of the layer below > 0] as bf16 into d.
+__device__ __forceinline__ void train_epilogue_delta(uint32_t t_row, const uint8_t* act, uint8_t* d, int r, int c0) {
+    float v[32];
+    tc::tmem_ld32(t_row + c0, v);
 #pragma unroll
-    for (int c = 0; c < kHid; c += 16) {
-        float v[16];
-        tc::tmem_ld16(t_row + c, v);
+    for (int j = 0; j < 32; j += 8) {
+        const uint4 m = *reinterpret_cast<const uint4*>(act + tc::kmajor_offset(r, c0 + j, 80));
+        const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
-        for (int j = 0; j < 16; j += 8) {
-            const uint4 m = *reinterpret_cast<const uint4*>(act + tc::kmajor_offset(r, c + j, 80));
-            const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&m);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v[j + q] = __bfloat162float(mb[q]) > 0.0f ? v[j + q] : 0.0f;
+        for (int q = 0; q < 4; ++q) {  // a bf16 is > 0 where its bits, as a signed number, are
+            v[j + 2 * q] = (int)(mw[q] << 16) > 0 ? v[j + 2 * q] : 0.0f;
+            v[j + 2 * q + 1] = (int)(mw[q] & 0xffff0000u) > 0 ? v[j + 2 * q + 1] : 0.0f;
         }
-        *reinterpret_cast<uint4*>(d + tc::kmajor_offset(r, c, 128)) = tc::pack8_bf16(v);
-        *reinterpret_cast<uint4*>(d + tc::kmajor_offset(r, c + 8, 128)) = tc::pack8_bf16(v + 8);
+        *reinterpret_cast<uint4*>(d + tc::kmajor_offset(r, c0 + j, kHid)) = tc::pack8_bf16(v + j);
     }
 }
 
 // Each CTA trains on tiles tile0 + blockIdx.x, + gridDim.x, ... and writes its gradient sum (and
-// its squared-error sum at index kParams) as row blockIdx.x of Gp (kParams + 1 floats per row);
+// its squared-error sum at index kParams) as row blockIdx.x of Gp (kRow floats per row);
 // the rows are summed by the Adam (or gradient) kernel, so no two CTAs write the same address.
-__global__ void __launch_bounds__(128, 2) train_kernel(const __nv_bfloat16* __restrict__ X, const float* __restrict__ T,
+__global__ void __launch_bounds__(256, 2) train_kernel(const __nv_bfloat16* __restrict__ X, const float* __restrict__ T,
                                                        int n, int tile0, int tiles, float inv_batch,
                                                        const float* __restrict__ P,
                                                        const __nv_bfloat16* __restrict__ WB, float* __restrict__ Gp_all,
                                                        int* status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
-    __shared__ float s_out[kHid + 2];  // w4 gradient, b4 gradient, loss of the CTA
-    float* Gp = Gp_all + (size_t)blockIdx.x * (kParams + 1);
-    if (threadIdx.x < kHid + 2) s_out[threadIdx.x] = 0.0f;
+    float* Gp = Gp_all + (size_t)blockIdx.x * kRow;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int quad = warp & 3, half = warp >> 2;  // a warp reads the TMEM lanes 32 (warp % 4) ..
+    const int r = quad * 32 + lane, c0 = half * 32;
     load_weights(S.w, P, WB);
     // Constant columns: ones (bias gradients) and zeros (padding), written once.
     {
-        const __nv_bfloat16 one = __float2bfloat16_rn(1.0f), zero = __float2bfloat16_rn(0.0f);
-        for (int c = 16; c < 32; ++c)
-            *reinterpret_cast<__nv_bfloat16*>(S.x + tc::kmajor_offset(tid, c, 32)) = c == 16 ? one : zero;
-        for (int c = 64; c < 80; ++c) {
-            *reinterpret_cast<__nv_bfloat16*>(S.h1 + tc::kmajor_offset(tid, c, 80)) = c == 64 ? one : zero;
-            *reinterpret_cast<__nv_bfloat16*>(S.h2 + tc::kmajor_offset(tid, c, 80)) = c == 64 ? one : zero;
-        }
-        for (int c = 64; c < 128; c += 8)
-            *reinterpret_cast<uint4*>(S.d + tc::kmajor_offset(tid, c, 128)) = make_uint4(0, 0, 0, 0);
+        const uint4 zero = make_uint4(0, 0, 0, 0), one = make_uint4(0x3f80u, 0, 0, 0);  // bf16 1 in column 0 of 8
+        uint8_t* xt = S.x[half];
+        *reinterpret_cast<uint4*>(xt + tc::kmajor_offset(r, 16, 32)) = one;
+        *reinterpret_cast<uint4*>(xt + tc::kmajor_offset(r, 24, 32)) = zero;
+        uint8_t* h = half ? S.h2 : S.h1;
+        *reinterpret_cast<uint4*>(h + tc::kmajor_offset(r, 64, 80)) = one;
+        *reinterpret_cast<uint4*>(h + tc::kmajor_offset(r, 72, 80)) = zero;
     }
     if (tid == 0) tc::mbar_init(&S.bar, 1);
     if (warp == 0) tc::tmem_alloc(&S.tslot, 256);
@@ -497,66 +524,89 @@ __global__ void __launch_bounds__(128, 2) train_kernel(const __nv_bfloat16* __re
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t taddr = S.tslot;
-    const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
     // Tensor-memory columns: activations / deltas (64), then the weight gradients of layers 3 and 2
     // (64 + bias + padding = 80 each) and 1 (16 + bias + padding = 32), summed over the CTA's tiles.
     const uint32_t tA = taddr, tW3 = taddr + 64, tW2 = taddr + 144, tW1 = taddr + 224;
-    const uint32_t sx = tc::smem_u32(S.x), sh1 = tc::smem_u32(S.h1), sh2 = tc::smem_u32(S.h2), sd = tc::smem_u32(S.d);
+    const uint32_t sh1 = tc::smem_u32(S.h1), sh2 = tc::smem_u32(S.h2);
+    const uint32_t sd0 = tc::smem_u32(S.d[0]), sd1 = tc::smem_u32(S.d[1]);
     const uint32_t idesc_fwd = tc::idesc_bf16(128, kHid);
-    uint32_t acc_dw = 0;  // 0 for the CTA's first tile: its gradient GEMMs overwrite the columns
     uint32_t phase = 0;
-    bool failed = false;
-    float acc_dw4[kHid];
+    bool bad = false;  // this thread's wait gave up; the CTA leaves together at the next phase
+    float acc_dw4[32];
 #pragma unroll
-    for (int j = 0; j < kHid; ++j) acc_dw4[j] = 0.0f;
+    for (int j = 0; j < 32; ++j) acc_dw4[j] = 0.0f;
     float acc_db4 = 0.0f, acc_loss = 0.0f;
 
-    // Issues one group of MMAs from thread 0 after the block's shared-memory writes, then waits.
-    auto run_mma = [&](auto&& issue) -> bool {
+    // One phase: after the block's shared-memory writes thread 0 issues `chain`, commits, and issues
+    // `beside`, which nothing waits for yet; every thread waits for the commit.  False: a wait gave up.
+    auto run_mma = [&](auto&& chain, auto&& beside) -> bool {
         tc::fence_async_smem();
         tc::fence_before_sync();
-        __syncthreads();
+        if (__syncthreads_or(bad)) return false;
         tc::fence_after_sync();
         if (tid == 0) {
-            issue();
+            chain();
             tc::mma_commit(&S.bar);
+            beside();
         }
-        const bool ok = tc::mbar_wait(&S.bar, phase);
+        bad = !tc::mbar_wait(&S.bar, phase);
         phase ^= 1u;
-        if (__syncthreads_or(!ok)) return false;
         tc::fence_after_sync();
         return true;
     };
+    auto nothing = [] {};
 
-    uint4 xa, xb;
+    uint4 xa;
     float tv;
-    load_sample(X, T, (tile0 + (int)blockIdx.x) * 128 + tid, n, xa, xb, tv);
-    for (int tile = tile0 + blockIdx.x; tile < tile0 + tiles && !failed; tile += gridDim.x) {
-        const int row = tile * 128 + tid;
+    load_sample(X, T, (tile0 + (int)blockIdx.x) * 128 + r, n, half, xa, tv);
+    int done = 0;  // tiles of this CTA behind the current one
+    bool ok = true;
+    for (int tile = tile0 + blockIdx.x; tile < tile0 + tiles; tile += gridDim.x, ++done) {
+        const int row = tile * 128 + r;
         const bool valid = row < n;
         const float target = tv;
-        *reinterpret_cast<uint4*>(S.x + tc::kmajor_offset(tid, 0, 32)) = xa;
-        *reinterpret_cast<uint4*>(S.x + tc::kmajor_offset(tid, 8, 32)) = xb;
-        if (tile + (int)gridDim.x < tile0 + tiles) load_sample(X, T, (tile + (int)gridDim.x) * 128 + tid, n, xa, xb, tv);
-        // ---- forward
-        if (!(failed = !run_mma([&] { gemm_kk(tA, sx, 32, tc::smem_u32(S.w.w1), kIn, kIn, kHid, idesc_fwd, 0u); }))) {
-            train_epilogue_hidden(tA + lane_off, S.w.b1, S.h1, tid);
-        }
-        if (failed) break;
-        if (!(failed = !run_mma([&] { gemm_kk(tA, sh1, 80, tc::smem_u32(S.w.w2), kHid, kHid, kHid, idesc_fwd, 0u); }))) {
-            train_epilogue_hidden(tA + lane_off, S.w.b2, S.h2, tid);
-        }
-        if (failed) break;
-        if ((failed = !run_mma([&] { gemm_kk(tA, sh2, 80, tc::smem_u32(S.w.w3), kHid, kHid, kHid, idesc_fwd, 0u); })))
-            break;
+        const uint32_t acc = done ? 1u : 0u;  // the CTA's first tile overwrites the gradient columns
+        uint8_t* xt = S.x[done & 1];
+        const uint32_t sx = tc::smem_u32(xt), sx_before = tc::smem_u32(S.x[(done & 1) ^ 1]);
+        *reinterpret_cast<uint4*>(xt + tc::kmajor_offset(r, 8 * half, 32)) = xa;
+        if (tile + (int)gridDim.x < tile0 + tiles) load_sample(X, T, (tile + (int)gridDim.x) * 128 + r, n, half, xa, tv);
+        // ---- forward; dW1 of the tile before beside the first layer
+        ok = run_mma([&] { gemm_kk(tA, sx, 32, tc::smem_u32(S.w.w1), kIn, kIn, kHid, idesc_fwd, 0u); },
+                     [&] {
+                         if (done) gemm_dw(tW1, sd0, sx_before, 32, done > 1 ? 1u : 0u);
+                     });
+        if (!ok) break;
+        train_epilogue_hidden(tA + lane_off, S.w.b1, S.h1, r, c0);
+        ok = run_mma([&] { gemm_kk(tA, sh1, 80, tc::smem_u32(S.w.w2), kHid, kHid, kHid, idesc_fwd, 0u); }, nothing);
+        if (!ok) break;
+        train_epilogue_hidden(tA + lane_off, S.w.b2, S.h2, r, c0);
+        ok = run_mma([&] { gemm_kk(tA, sh2, 80, tc::smem_u32(S.w.w3), kHid, kHid, kHid, idesc_fwd, 0u); }, nothing);
+        if (!ok) break;
         // ---- output layer, loss, and the output-layer delta (CUDA cores)
+        // z is summed over the 64 columns in order by both threads of a row; each keeps its own half of h3.
+        float v[32];
         float z = S.w.b4;
+        auto columns = [&](int c, float* h) {
+            tc::tmem_ld16(tA + lane_off + c, h);
 #pragma unroll
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tc::tmem_ld16(tA + lane_off + c, v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) z += fmaxf(v[j] + S.w.b3[c + j], 0.0f) * S.w.w4[c + j];
+            for (int j = 0; j < 16; ++j) {
+                h[j] = fmaxf(h[j] + S.w.b3[c + j], 0.0f);
+                z += h[j] * S.w.w4[c + j];
+            }
+        };
+        if (half == 0) {
+            float other[16];
+            columns(0, v);
+            columns(16, v + 16);
+            columns(32, other);
+            columns(48, other);
+        } else {
+            float other[16];
+            columns(0, other);
+            columns(16, other);
+            columns(32, v);
+            columns(48, v + 16);
         }
         const float y = 1.0f / (1.0f + expf(-z));
         const float err = valid ? y - target : 0.0f;
@@ -564,91 +614,105 @@ __global__ void __launch_bounds__(128, 2) train_kernel(const __nv_bfloat16* __re
         acc_loss += err * err;
         acc_db4 += dz;
 #pragma unroll
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tc::tmem_ld16(tA + lane_off + c, v);
+        for (int j = 0; j < 32; j += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(S.w.w4 + c0 + j);
+            const float wj[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float h = fmaxf(v[j] + S.w.b3[c + j], 0.0f);
-                acc_dw4[c + j] += dz * h;
-                v[j] = h > 0.0f ? dz * S.w.w4[c + j] : 0.0f;
+            for (int q = 0; q < 4; ++q) {
+                acc_dw4[j + q] += dz * v[j + q];
+                v[j + q] = v[j + q] > 0.0f ? dz * wj[q] : 0.0f;
             }
-            *reinterpret_cast<uint4*>(S.d + tc::kmajor_offset(tid, c, 128)) = tc::pack8_bf16(v);
-            *reinterpret_cast<uint4*>(S.d + tc::kmajor_offset(tid, c + 8, 128)) = tc::pack8_bf16(v + 8);
         }
-        // ---- layer 3: dW3 and the delta of layer 2
-        if (!(failed = !run_mma([&] {
-                  gemm_dw(tW3, sd, sh2, 80, acc_dw);
-                  gemm_delta(tA, sd, tc::smem_u32(S.w.w3));
-              }))) {
-            train_epilogue_delta(tA + lane_off, S.h2, S.d, tid);
-        }
-        if (failed) break;
-        // ---- layer 2: dW2 and the delta of layer 1
-        if (!(failed = !run_mma([&] {
-                  gemm_dw(tW2, sd, sh1, 80, acc_dw);
-                  gemm_delta(tA, sd, tc::smem_u32(S.w.w2));
-              }))) {
-            train_epilogue_delta(tA + lane_off, S.h1, S.d, tid);
-        }
-        if (failed) break;
-        // ---- layer 1: dW1
-        if ((failed = !run_mma([&] { gemm_dw(tW1, sd, sx, 32, acc_dw); }))) break;
-        acc_dw = 1u;
-    }
-    // ---- hidden-layer weight gradients of all the CTA's tiles
-    if (!failed && acc_dw && warp < 2) {
-        const int o = warp * 32 + lane;
-        flush_dw(tW3 + lane_off, o, kHid, Gp, OFF_W3, OFF_B3);
-        flush_dw(tW2 + lane_off, o, kHid, Gp, OFF_W2, OFF_B2);
-        flush_dw(tW1 + lane_off, o, kIn, Gp, OFF_W1, OFF_B1);
-    }
-    // ---- output-layer gradients and loss: warp sums, then the CTA's sum
 #pragma unroll
-    for (int j = 0; j < kHid; ++j) {
-        const float v = warp_sum(acc_dw4[j]);
-        if (lane == 0) atomicAdd(&s_out[j], v);
+        for (int j = 0; j < 32; j += 8)
+            *reinterpret_cast<uint4*>(S.d[0] + tc::kmajor_offset(r, c0 + j, kHid)) = tc::pack8_bf16(v + j);
+        // ---- the delta of layer 2, dW3 beside its epilogue
+        ok = run_mma([&] { gemm_delta(tA, sd0, tc::smem_u32(S.w.w3)); }, [&] { gemm_dw(tW3, sd0, sh2, 80, acc); });
+        if (!ok) break;
+        train_epilogue_delta(tA + lane_off, S.h2, S.d[1], r, c0);
+        // ---- the delta of layer 1, dW2 beside its epilogue (d[0] is free: this wait covers dW3)
+        ok = run_mma([&] { gemm_delta(tA, sd1, tc::smem_u32(S.w.w2)); }, [&] { gemm_dw(tW2, sd1, sh1, 80, acc); });
+        if (!ok) break;
+        train_epilogue_delta(tA + lane_off, S.h1, S.d[0], r, c0);
     }
+    if (ok && done) {  // dW1 of the last tile, and all before it
+        ok = run_mma([&] { gemm_dw(tW1, sd0, tc::smem_u32(S.x[(done & 1) ^ 1]), 32, done > 1 ? 1u : 0u); }, nothing);
+    }
+    // ---- output-layer gradients and loss: sums over 32 rows, then over the CTA's four groups of them
     {
-        const float v = warp_sum(acc_db4), l2 = warp_sum(acc_loss);
-        if (lane == 0) {
-            atomicAdd(&s_out[kHid], v);
-            atomicAdd(&s_out[kHid + 1], l2);
+        const float v = warp_sum32(acc_dw4);
+        S.out[quad][c0 + lane] = v;
+        const float db = warp_sum(acc_db4), l2 = warp_sum(acc_loss);
+        if (half == 0 && lane == 0) {
+            S.out[quad][kHid] = db;
+            S.out[quad][kHid + 1] = l2;
         }
     }
-    __syncthreads();
-    if (tid < kHid) Gp[OFF_W4 + tid] = s_out[tid];
-    if (tid == kHid) Gp[OFF_B4] = s_out[kHid];
-    if (tid == kHid + 1) Gp[kParams] = s_out[kHid + 1];
+    const bool failed = __syncthreads_or(bad || !ok) != 0;
+    // ---- hidden-layer weight gradients of all the CTA's tiles
+    if (!failed && done && quad < 2) {
+        const int o = quad * 32 + lane;
+        flush_dw(tW3 + lane_off, o, kHid, half * 48, half ? 80 : 48, Gp, OFF_W3, OFF_B3);
+        flush_dw(tW2 + lane_off, o, kHid, half ? 0 : 32, half ? 32 : 80, Gp, OFF_W2, OFF_B2);
+        flush_dw(tW1 + lane_off, o, kIn, half * 16, half ? 32 : 16, Gp, OFF_W1, OFF_B1);
+    }
+    if (tid < kHid + 2) {
+        const float g = ((S.out[2][tid] + S.out[3][tid]) + S.out[1][tid]) + S.out[0][tid];
+        Gp[tid < kHid ? OFF_W4 + tid : (tid == kHid ? OFF_B4 : kParams)] = g;
+    }
     if (failed && tid == 0) atomicExch(status, 1);
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(taddr, 256);
 }
 
-// Adam on the FP32 parameters; refreshes the BF16 copies and clears the gradient buffer.
-// Sum of the training kernel's `parts` partial rows at index i (i == kParams: the squared error).
+// Sum of the training kernel's `parts` partial rows, in row order, at index i (i == kParams: the squared
+// error), for the 32 indices of a block of 8 warps; valid in the first warp.  The warps fetch the rows
+// side by side into shared memory and the first one adds them up: one thread per index over all rows was a
+// chain of loads, 17.7 us for 304 rows against 12.4 (under ncu, cold caches), the same sums.
+constexpr int kRowsAtOnce = 320;
 __device__ __forceinline__ float sum_parts(const float* __restrict__ Gp, int parts, int i) {
+    __shared__ float s_rows[kRowsAtOnce][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
     float g = 0.0f;
-    for (int c = 0; c < parts; ++c) g += Gp[(size_t)c * (kParams + 1) + i];
+    for (int c0 = 0; c0 < parts; c0 += kRowsAtOnce) {
+        const int rows = min(parts - c0, kRowsAtOnce);
+        if (c0) __syncthreads();
+        if (i <= kParams) {
+#pragma unroll 10
+            for (int c = slice; c < rows; c += 8) s_rows[c][lane] = __ldcg(Gp + (size_t)(c0 + c) * kRow + i);
+        }
+        __syncthreads();
+        if (slice == 0 && i <= kParams) {
+#pragma unroll 16
+            for (int c = 0; c < rows; ++c) g += s_rows[c][lane];
+        }
+    }
     return g;
 }
 
+constexpr int kSumBlocks = (kParams + 1 + 31) / 32;  // of 256 threads, for the two kernels below
+
 // Gradient (and loss) of a training launch into G and *loss, for callers that read the gradient.
-__global__ void reduce_grad_kernel(const float* __restrict__ Gp, int parts, float* __restrict__ G,
-                                   float* __restrict__ loss) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kParams) G[i] = sum_parts(Gp, parts, i);
-    if (i == kParams && loss) *loss = sum_parts(Gp, parts, i);
+__global__ void __launch_bounds__(256) reduce_grad_kernel(const float* __restrict__ Gp, int parts, float* __restrict__ G,
+                                                          float* __restrict__ loss) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float g = sum_parts(Gp, parts, i);
+    if (threadIdx.x >= 32) return;
+    if (i < kParams) G[i] = g;
+    if (i == kParams && loss) *loss = g;
 }
 
-__global__ void adam_kernel(float* __restrict__ P, __nv_bfloat16* __restrict__ WB, const float* __restrict__ Gp,
-                            int parts, float* __restrict__ loss, float* __restrict__ Mo, float* __restrict__ Vo,
-                            float lr, float b1, float b2, float eps, float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == kParams && loss) *loss = sum_parts(Gp, parts, i);
-    if (i >= kParams) return;
+// Adam on the FP32 parameters; refreshes the BF16 copies.
+__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ P, __nv_bfloat16* __restrict__ WB,
+                                                   const float* __restrict__ Gp, int parts, float* __restrict__ loss,
+                                                   float* __restrict__ Mo, float* __restrict__ Vo, float lr, float b1,
+                                                   float b2, float eps, float c1, float c2) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
     const float g = sum_parts(Gp, parts, i);
+    if (threadIdx.x >= 32) return;
+    if (i == kParams && loss) *loss = g;
+    if (i >= kParams) return;
     const float m = b1 * Mo[i] + (1.0f - b1) * g;
     const float v = b2 * Vo[i] + (1.0f - b2) * g * g;
     Mo[i] = m;
@@ -728,7 +792,7 @@ int train_grid(mm_mlp m, int tiles) { return tiles < 2 * m->num_sms ? tiles : 2 
 int run_train(mm_mlp m, const void* X, const float* T, int n, int tile0, int tiles, float inv_batch, cudaStream_t s) {
     const int grid = train_grid(m, tiles);
     // The shared-memory image needs 1024-byte alignment; the kernel takes the dynamic buffer as is.
-    mm::mlp::train_kernel<<<grid, 128, train_smem(), s>>>((const __nv_bfloat16*)X, T, n, tile0, tiles, inv_batch, m->P,
+    mm::mlp::train_kernel<<<grid, 256, train_smem(), s>>>((const __nv_bfloat16*)X, T, n, tile0, tiles, inv_batch, m->P,
                                                          m->WB, m->Gp, m->status);
     MM_CUDA_TRY(cudaGetLastError());
     mm::count_launch();
@@ -776,7 +840,7 @@ int mm_mlp_create(uint32_t seed, mm_mlp* out) {
     cudaError_t e = cudaSuccess;
     e = e ? e : cudaMalloc(&m->P, kParams * sizeof(float));
     e = e ? e : cudaMalloc(&m->WB, kBf16 * sizeof(__nv_bfloat16));
-    e = e ? e : cudaMalloc(&m->Gp, (size_t)2 * m->num_sms * (kParams + 1) * sizeof(float));
+    e = e ? e : cudaMalloc(&m->Gp, (size_t)2 * m->num_sms * kRow * sizeof(float));
     e = e ? e : cudaMalloc(&m->M, kParams * sizeof(float));
     e = e ? e : cudaMalloc(&m->V, kParams * sizeof(float));
     e = e ? e : cudaMalloc(&m->loss, sizeof(float));
@@ -864,7 +928,7 @@ int mm_mlp_gradients(mm_mlp m, const void* d_x, const float* d_t, int n, float* 
     cudaStream_t s = (cudaStream_t)stream;
     const int tiles = (n + 127) / 128;
     if ((r = run_train(m, d_x, d_t, n, 0, tiles, 1.0f / (float)n, s))) return r;
-    mm::mlp::reduce_grad_kernel<<<(mm::mlp::kParams + 256) / 256, 256, 0, s>>>(m->Gp, train_grid(m, tiles), d_grad,
+    mm::mlp::reduce_grad_kernel<<<mm::mlp::kSumBlocks, 256, 0, s>>>(m->Gp, train_grid(m, tiles), d_grad,
                                                                               m->loss);
     MM_CUDA_TRY(cudaGetLastError());
     mm::count_launch();
@@ -895,7 +959,7 @@ int mm_mlp_train(mm_mlp m, const void* d_x, const float* d_t, int n, int batch, 
         cursor += tiles;
         m->step += 1;
         const float c1 = 1.0f - powf(b1, (float)m->step), c2 = 1.0f - powf(b2, (float)m->step);
-        mm::mlp::adam_kernel<<<(mm::mlp::kParams + 256) / 256, 256, 0, s>>>(
+        mm::mlp::adam_kernel<<<mm::mlp::kSumBlocks, 256, 0, s>>>(
             m->P, m->WB, m->Gp, train_grid(m, tiles), h_loss_history ? m->loss : nullptr, m->M, m->V, lr, b1, b2, eps,
             c1, c2);
         MM_CUDA_TRY(cudaGetLastError());
