@@ -184,23 +184,24 @@ struct SmemWeights {
 };
 
 __device__ void load_weights(SmemWeights& sw, const float* __restrict__ P, const __nv_bfloat16* __restrict__ WB) {
-    // 8 consecutive inputs of one output row are one 16-byte core-matrix row: one vector copy each.
+    // 8 consecutive inputs of one output row are one 16-byte core-matrix row: one vector copy each.  From
+    // L2: the optimizer may write them after this kernel has started (launch_behind).
     const uint4* wb = reinterpret_cast<const uint4*>(WB);
     for (int i = threadIdx.x; i < kHid * kIn / 8; i += blockDim.x)
         *reinterpret_cast<uint4*>(sw.w1 + tc::kmajor_offset(i / (kIn / 8), (i % (kIn / 8)) * 8, kIn)) =
-            __ldg(wb + OFFB_W1 / 8 + i);
+            __ldcg(wb + OFFB_W1 / 8 + i);
     for (int i = threadIdx.x; i < kHid * kHid / 8; i += blockDim.x) {
         const int o = i / (kHid / 8), k = (i % (kHid / 8)) * 8;
-        *reinterpret_cast<uint4*>(sw.w2 + tc::kmajor_offset(o, k, kHid)) = __ldg(wb + OFFB_W2 / 8 + i);
-        *reinterpret_cast<uint4*>(sw.w3 + tc::kmajor_offset(o, k, kHid)) = __ldg(wb + OFFB_W3 / 8 + i);
+        *reinterpret_cast<uint4*>(sw.w2 + tc::kmajor_offset(o, k, kHid)) = __ldcg(wb + OFFB_W2 / 8 + i);
+        *reinterpret_cast<uint4*>(sw.w3 + tc::kmajor_offset(o, k, kHid)) = __ldcg(wb + OFFB_W3 / 8 + i);
     }
     for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
-        sw.b1[i] = P[OFF_B1 + i];
-        sw.b2[i] = P[OFF_B2 + i];
-        sw.b3[i] = P[OFF_B3 + i];
-        sw.w4[i] = P[OFF_W4 + i];
+        sw.b1[i] = __ldcg(P + OFF_B1 + i);
+        sw.b2[i] = __ldcg(P + OFF_B2 + i);
+        sw.b3[i] = __ldcg(P + OFF_B3 + i);
+        sw.w4[i] = __ldcg(P + OFF_W4 + i);
     }
-    if (threadIdx.x == 0) sw.b4 = P[OFF_B4];
+    if (threadIdx.x == 0) sw.b4 = __ldcg(P + OFF_B4);
 }
 
 // ------------------------------------------------------------------------------ inference
@@ -366,6 +367,30 @@ __global__ void __launch_bounds__(128, 5) infer_kernel(const __nv_bfloat16* __re
 // One Adam step at batch 131,072, this kernel: 48.4 us with 128 threads a CTA, a weight-gradient GEMM on the
 // chain and six waits of two barriers -> 28.1 us (both under ncu).  The hidden layers' gradients keep every bit.
 
+// Launches of a training run follow each other without a gap: a kernel launched with launch_behind may
+// start when every CTA of the one before has called grid_trigger (or ended), and sees that kernel's writes
+// after grid_wait.  The training kernel of a step sets up its tiles while Adam of the step before runs;
+// samples are read before the wait, since no kernel of a run writes them.  8 steps at batch 131,072 and
+// 262,144 predictions take 322 us against 346, 8 steps at batch 16,384 and 40,000 predictions 161 against 185.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_behind(bool behind, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t s,
+                          Args... args) {
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a[0].val.programmaticStreamSerializationAllowed = 1;
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = a;
+    c.numAttrs = behind ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+}
+
 struct TrainSmem {
     alignas(128) uint8_t x[2][128 * 32 * 2];
     alignas(128) uint8_t h1[128 * 80 * 2];
@@ -507,7 +532,6 @@ __global__ void __launch_bounds__(256, 2) train_kernel(const __nv_bfloat16* __re
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, half = warp >> 2;  // a warp reads the TMEM lanes 32 (warp % 4) ..
     const int r = quad * 32 + lane, c0 = half * 32;
-    load_weights(S.w, P, WB);
     // Constant columns: ones (bias gradients) and zeros (padding), written once.
     {
         const uint4 zero = make_uint4(0, 0, 0, 0), one = make_uint4(0x3f80u, 0, 0, 0);  // bf16 1 in column 0 of 8
@@ -518,8 +542,13 @@ __global__ void __launch_bounds__(256, 2) train_kernel(const __nv_bfloat16* __re
         *reinterpret_cast<uint4*>(h + tc::kmajor_offset(r, 64, 80)) = one;
         *reinterpret_cast<uint4*>(h + tc::kmajor_offset(r, 72, 80)) = zero;
     }
+    uint4 xa;
+    float tv;
+    load_sample(X, T, (tile0 + (int)blockIdx.x) * 128 + r, n, half, xa, tv);
     if (tid == 0) tc::mbar_init(&S.bar, 1);
     if (warp == 0) tc::tmem_alloc(&S.tslot, 256);
+    grid_wait();  // the parameters of the step before
+    load_weights(S.w, P, WB);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -557,9 +586,6 @@ __global__ void __launch_bounds__(256, 2) train_kernel(const __nv_bfloat16* __re
     };
     auto nothing = [] {};
 
-    uint4 xa;
-    float tv;
-    load_sample(X, T, (tile0 + (int)blockIdx.x) * 128 + r, n, half, xa, tv);
     int done = 0;  // tiles of this CTA behind the current one
     bool ok = true;
     for (int tile = tile0 + blockIdx.x; tile < tile0 + tiles; tile += gridDim.x, ++done) {
@@ -638,6 +664,7 @@ __global__ void __launch_bounds__(256, 2) train_kernel(const __nv_bfloat16* __re
     if (ok && done) {  // dW1 of the last tile, and all before it
         ok = run_mma([&] { gemm_dw(tW1, sd0, tc::smem_u32(S.x[(done & 1) ^ 1]), 32, done > 1 ? 1u : 0u); }, nothing);
     }
+    grid_trigger();  // the kernel that sums the rows may take its place
     // ---- output-layer gradients and loss: sums over 32 rows, then over the CTA's four groups of them
     {
         const float v = warp_sum32(acc_dw4);
@@ -709,6 +736,8 @@ __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ P, __nv_b
                                                    float* __restrict__ Mo, float* __restrict__ Vo, float lr, float b1,
                                                    float b2, float eps, float c1, float c2) {
     const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    grid_trigger();
+    grid_wait();
     const float g = sum_parts(Gp, parts, i);
     if (threadIdx.x >= 32) return;
     if (i == kParams && loss) *loss = g;
@@ -788,13 +817,15 @@ int refresh(mm_mlp m, cudaStream_t s) {
 // Partial-gradient rows of a training launch over `tiles` tiles: two CTAs per SM, each at least one tile.
 int train_grid(mm_mlp m, int tiles) { return tiles < 2 * m->num_sms ? tiles : 2 * m->num_sms; }
 
-// Runs the training kernel over tiles [tile0, tile0 + tiles) of (X, T) into m->Gp (train_grid rows).
-int run_train(mm_mlp m, const void* X, const float* T, int n, int tile0, int tiles, float inv_batch, cudaStream_t s) {
+// Runs the training kernel over tiles [tile0, tile0 + tiles) of (X, T) into m->Gp (train_grid rows);
+// `behind`: the kernel before it on the stream is the run's own (launch_behind).
+int run_train(mm_mlp m, const void* X, const float* T, int n, int tile0, int tiles, float inv_batch, bool behind,
+              cudaStream_t s) {
     const int grid = train_grid(m, tiles);
     // The shared-memory image needs 1024-byte alignment; the kernel takes the dynamic buffer as is.
-    mm::mlp::train_kernel<<<grid, 256, train_smem(), s>>>((const __nv_bfloat16*)X, T, n, tile0, tiles, inv_batch, m->P,
-                                                         m->WB, m->Gp, m->status);
-    MM_CUDA_TRY(cudaGetLastError());
+    MM_CUDA_TRY(mm::mlp::launch_behind(behind, mm::mlp::train_kernel, grid, 256, train_smem(), s,
+                                       (const __nv_bfloat16*)X, T, n, tile0, tiles, inv_batch, m->P, m->WB, m->Gp,
+                                       m->status));
     mm::count_launch();
     return MM_OK;
 }
@@ -927,7 +958,7 @@ int mm_mlp_gradients(mm_mlp m, const void* d_x, const float* d_t, int n, float* 
     if (r) return r;
     cudaStream_t s = (cudaStream_t)stream;
     const int tiles = (n + 127) / 128;
-    if ((r = run_train(m, d_x, d_t, n, 0, tiles, 1.0f / (float)n, s))) return r;
+    if ((r = run_train(m, d_x, d_t, n, 0, tiles, 1.0f / (float)n, false, s))) return r;
     mm::mlp::reduce_grad_kernel<<<mm::mlp::kSumBlocks, 256, 0, s>>>(m->Gp, train_grid(m, tiles), d_grad,
                                                                               m->loss);
     MM_CUDA_TRY(cudaGetLastError());
@@ -955,14 +986,13 @@ int mm_mlp_train(mm_mlp m, const void* d_x, const float* d_t, int n, int batch, 
     int cursor = 0;
     for (int k = 0; k < steps; ++k) {
         if (cursor + tiles > total_tiles) cursor = 0;
-        if ((r = run_train(m, d_x, d_t, n, cursor, tiles, 1.0f / (float)(tiles * 128), s))) return r;
+        if ((r = run_train(m, d_x, d_t, n, cursor, tiles, 1.0f / (float)(tiles * 128), k > 0 && !h_loss_history, s))) return r;
         cursor += tiles;
         m->step += 1;
         const float c1 = 1.0f - powf(b1, (float)m->step), c2 = 1.0f - powf(b2, (float)m->step);
-        mm::mlp::adam_kernel<<<mm::mlp::kSumBlocks, 256, 0, s>>>(
-            m->P, m->WB, m->Gp, train_grid(m, tiles), h_loss_history ? m->loss : nullptr, m->M, m->V, lr, b1, b2, eps,
-            c1, c2);
-        MM_CUDA_TRY(cudaGetLastError());
+        MM_CUDA_TRY(mm::mlp::launch_behind(true, mm::mlp::adam_kernel, mm::mlp::kSumBlocks, 256, 0, s, m->P, m->WB, m->Gp,
+                                           train_grid(m, tiles), h_loss_history ? m->loss : nullptr, m->M, m->V, lr, b1,
+                                           b2, eps, c1, c2));
         mm::count_launch();
         if (h_loss_history) {
             float l = 0.0f;
