@@ -42,6 +42,7 @@ struct P {
     size_t dst_depth_pitch;
     int width, height;
     int skip_phase;  // >= 0: leave the pixels of this 1/16 phase alone
+    int src_row;      // src_pitch in texels; 0: the image needs 64-bit texel indices
 };
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
@@ -50,8 +51,13 @@ __device__ __forceinline__ float4 texel(const P& p, int x, int y) {
     return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const char*>(p.src) + (size_t)y * p.src_pitch) + x);
 }
 
-__global__ void __launch_bounds__(256) reproject_fast_kernel(P p) {
-    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+// 128 threads and 16 blocks an SM (32 registers): the fetches wait for L2 (44% of them hit L1 at a motion of
+// 100 pixels), and warps in flight hide it better than fetches in flight do.  2880x1620 with a turn of 4
+// degrees / 3840x2160 with 0.5: 6 blocks of 256 threads 64.0 / 103.7 us, 4 (50 registers) 77.6 / 129.9, 8
+// 54.9 / 87.0, 16 blocks of 32 x 4 53.3 / 84.6, 4 of 32 x 16 57.9 / 92.1.
+constexpr int kBlockW = 32, kBlockH = 4;
+__global__ void __launch_bounds__(kBlockW * kBlockH, 16) reproject_fast_kernel(P p) {
+    const int x = blockIdx.x * kBlockW + threadIdx.x, y = blockIdx.y * kBlockH + threadIdx.y;
     if (x >= p.width || y >= p.height) return;
     if (p.skip_phase >= 0 && (x & 3) == (p.skip_phase & 3) && (y & 3) == (p.skip_phase >> 2)) return;
     const float sx = fmaf((float)x, p.sxs, -1.0f), sy = fmaf((float)y, p.sys, -1.0f);
@@ -88,20 +94,47 @@ __global__ void __launch_bounds__(256) reproject_fast_kernel(P p) {
     const float W = (float)p.width, H = (float)p.height;
     const float ou = oldU * W, ov = oldV * H;
     const float bu = (oldU - (float)x * p.iw) * W, bv = (oldV - (float)y * p.ih) * H;
-    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // The taps lie on a line from (ou + bu / 2, ov + bv / 2) to (ou - bu / 2, ov - bv / 2), and rounding keeps
+    // their order along it, so with both ends inside the image no tap needs a clamp.  Then adding 1.5 * 2^23
+    // leaves the nearest integer (ties to even, as __float2int_rn) in the sum's low bits, and a texel is one
+    // multiply-add away: 44 M warp instructions instead of 51 M at 2880x1620, 64.1 -> 62.0 us by itself.
+    float sr = 0.0f, sg = 0.0f, sb = 0.0f, alpha;
+    int cx, cy;
+    const float u0 = fmaf(-bu, -0.5f, ou), u1 = fmaf(-bu, 0.5f, ou), v0 = fmaf(-bv, -0.5f, ov), v1 = fmaf(-bv, 0.5f, ov);
+    if (p.src_row && fminf(u0, u1) >= 0.0f && fmaxf(u0, u1) <= W - 1.0f && fminf(v0, v1) >= 0.0f &&
+        fmaxf(v0, v1) <= H - 1.0f) {
+        constexpr float kMagic = 12582912.0f;
+        constexpr unsigned kBits = 0x4B400000u;
+        const unsigned row = (unsigned)p.src_row, origin = kBits * row + kBits;  // modulo 2^32, as the sums below
 #pragma unroll
-    for (int s = 0; s < 10; ++s) {
-        const float k = (float)s / 9.0f - 0.5f;
-        const int tx = clampi(__float2int_rn(fmaf(-bu, k, ou)), 0, p.width - 1);
-        const int ty = clampi(__float2int_rn(fmaf(-bv, k, ov)), 0, p.height - 1);
-        const float4 t = texel(p, tx, ty);
-        acc.x += t.x;
-        acc.y += t.y;
-        acc.z += t.z;
-        acc.w += t.w;
+        for (int s = 0; s < 10; ++s) {
+            const float k = (float)s / 9.0f - 0.5f;
+            const unsigned tx = __float_as_uint(fmaf(-bu, k, ou) + kMagic), ty = __float_as_uint(fmaf(-bv, k, ov) + kMagic);
+            const float4 t = __ldg(p.src + (ty * row + tx - origin));
+            sr += t.x;
+            sg += t.y;
+            sb += t.z;
+        }
+        const unsigned mx = __float_as_uint(ou + kMagic), my = __float_as_uint(ov + kMagic);
+        alpha = __ldg(&(p.src + (my * row + mx - origin))->w);
+        cx = (int)(mx - kBits);
+        cy = (int)(my - kBits);
+    } else {
+#pragma unroll
+        for (int s = 0; s < 10; ++s) {
+            const float k = (float)s / 9.0f - 0.5f;
+            const int tx = clampi(__float2int_rn(fmaf(-bu, k, ou)), 0, p.width - 1);
+            const int ty = clampi(__float2int_rn(fmaf(-bv, k, ov)), 0, p.height - 1);
+            const float4 t = texel(p, tx, ty);
+            sr += t.x;
+            sg += t.y;
+            sb += t.z;
+        }
+        cx = clampi(__float2int_rn(ou), 0, p.width - 1);
+        cy = clampi(__float2int_rn(ov), 0, p.height - 1);
+        alpha = texel(p, cx, cy).w;
     }
-    const int cx = clampi(__float2int_rn(ou), 0, p.width - 1), cy = clampi(__float2int_rn(ov), 0, p.height - 1);
-    float4 o = make_float4(acc.x * 0.1f, acc.y * 0.1f, acc.z * 0.1f, texel(p, cx, cy).w);
+    const float4 o = make_float4(sr * 0.1f, sg * 0.1f, sb * 0.1f, alpha);
     *(reinterpret_cast<float4*>(reinterpret_cast<char*>(p.dst) + (size_t)y * p.dst_pitch) + x) = o;
     if (p.dst_depth && p.src_depth)
         *(reinterpret_cast<float*>(reinterpret_cast<char*>(p.dst_depth) + (size_t)y * p.dst_depth_pitch) + x) =
@@ -153,7 +186,11 @@ int launch_reproject_fast(const mm_uniforms& u, const mm_image& src, const mm_im
     p.width = dst.width;
     p.height = dst.height;
     p.skip_phase = skip_phase;
-    repf::reproject_fast_kernel<<<dim3((p.width + 31) / 32, (p.height + 7) / 8), dim3(32, 8), 0, s>>>(p);
+    const size_t row = src.rgba_pitch_bytes / 16;
+    p.src_row = row * (size_t)src.height < ((size_t)1 << 31) ? (int)row : 0;
+    const dim3 block(repf::kBlockW, repf::kBlockH);
+    const dim3 grid((p.width + block.x - 1) / block.x, (p.height + block.y - 1) / block.y);
+    repf::reproject_fast_kernel<<<grid, block, 0, s>>>(p);
     MM_CUDA_TRY(cudaGetLastError());
     count_launch();
     return MM_OK;
