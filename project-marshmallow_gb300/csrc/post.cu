@@ -176,6 +176,8 @@ static int post_pass(mm_context ctx, const mm_uniforms* u, const mm_image* src, 
     p.width = src->width;
     p.height = src->height;
     p.bgra = o.bgra;
+    const size_t row = src->rgba_pitch_bytes / 4;
+    p.src_row = row * (size_t)src->height < ((size_t)1 << 31) ? (int)row : 0;
     fill_constants(u, &p);
     return run(p, which, o.math, (cudaStream_t)stream);
 }
