@@ -1033,7 +1033,8 @@ struct ConePool {
 
 // One round: the `take` (<= 32) oldest records of the warp's pool, one per lane, then each owner's
 // blends in pool order.  Every lane of the warp calls it with the same head and take.
-template <bool E, int S>
+// Cone taps a lane issues together: G.
+template <bool E, int S, int G>
 __device__ __forceinline__ void cone_round(const MarchLaunch& p, const Frame& f, const V3* cone, ConePool& q,
                                            int head, int take, V3 rd, float& trans, float cosTheta, float hg,
                                            Work& w) {
@@ -1054,12 +1055,12 @@ __device__ __forceinline__ void cone_round(const MarchLaunch& p, const Frame& f,
         float dal = 0.0f;
         if constexpr (!E && MM_POOL_PARAM_CONE) {
 #pragma unroll
-            for (int i = 0; i < 6; i += MM_POOL_CONE_GROUP)
-                dal = cone_taps<E, S, MM_POOL_CONE_GROUP, true>(p, f, cone, i, pos, stepSize, dal, w.test, w.hires);
+            for (int i = 0; i < 6; i += G)
+                dal = cone_taps<E, S, G, true>(p, f, cone, i, pos, stepSize, dal, w.test, w.hires);
         } else {
 #pragma unroll 1
-            for (int i = 0; i < 6; i += MM_POOL_CONE_GROUP)
-                dal = cone_taps<E, S, MM_POOL_CONE_GROUP>(p, f, cone, i, pos, stepSize, dal, w.test, w.hires);
+            for (int i = 0; i < 6; i += G)
+                dal = cone_taps<E, S, G>(p, f, cone, i, pos, stepSize, dal, w.test, w.hires);
         }
         q.t[wp][slot] = shade_term<E>(dal, q.lm[wp][slot].lo, rh, cosO, hgO);
     }
@@ -1167,13 +1168,13 @@ __device__ __forceinline__ void march_pixel_q(const MarchLaunch& p, const Frame&
         const unsigned sum = __reduce_add_sync(full, (pushed ? 1u : 0u) + (alive ? 64u : 0u));
         pending += (int)(sum & 63u);
         if (pending >= 32) {  // < 64 records: < 32 after a round, at most 32 appended since
-            cone_round<E, S>(p, f, cone, q, head, 32, r.rd, trans, r.cosTheta, r.hg, w);
+            cone_round<E, S, MM_POOL_CONE_GROUP>(p, f, cone, q, head, 32, r.rd, trans, r.cosTheta, r.hg, w);
             head += 32;
             pending -= 32;
         }
         if (sum < 64u) break;
     }
-    if (pending > 0) cone_round<E, S>(p, f, cone, q, head, pending, r.rd, trans, r.cosTheta, r.hg, w);
+    if (pending > 0) cone_round<E, S, MM_POOL_CONE_GROUP>(p, f, cone, q, head, pending, r.rd, trans, r.cosTheta, r.hg, w);
     if (live) store_pixel(p, px, py, composite<E>(p.u, f, r.rd, r.bg, r.alpha, accum, trans), firstT);
 }
 
@@ -1246,7 +1247,7 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PAIR_MIN_BLOCKS) march
 // lanes marches one ray.  In a round, member j evaluates the sample the shader's loop would
 // reach j iterations later if nothing changed the step size or the mode: position t + s + ... + s
 // (j additions, as the loop's increments make it), its cloudTest, and in small-step mode its
-// cloudHiRes, sun cone and shading term where the shader would compute them.  The team then runs
+// cloudHiRes where the shader would compute it.  The team then runs
 // the loop body (:408-482) on the round's results in order, every member the same state; a step back
 // (:426-434) or a return to large steps (:468-474) changes the step size, so the rest of the round is
 // dropped and the next round starts where the loop goes on.  Every consumed sample is the computation
@@ -1257,25 +1258,24 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PAIR_MIN_BLOCKS) march
 // rays, ~300 us one thread per ray; a team of n lanes makes that chain shorter, but costs lanes: each
 // member sets the ray up, and a round's tail is dropped at every step-size change.  The more rays, the
 // smaller the teams; past ~600,000 rays the pooled kernel's throughput wins.  Cone taps in groups of G
-// at B blocks per SM: a larger G is faster for a ray, a larger B for the launch.  Microseconds on GB300,
+// at B blocks per SM: a larger G shortens a cone round, a larger B helps the launch.  Microseconds on GB300,
 // pitch 12, two seeds, whole images and (f) frames with 1 pixel in 16 marched (the reprojection beside):
-//   rays         36k    65k    76k    90k   153k   256k   331k   412k   518k   589k  704k   f129k  f518k
-//   8 G3 B6     71.8   82.7  100.0  118.1  171.9  268.2  338.6  414.9  508.2  570.1  664.8  175.2  600.3
-//   4 G3 B6    107.8  110.0  118.7  117.6  147.3  223.0  276.0  334.6  406.7  452.5  525.6  155.7  491.3
-//   4 G3 B7    111.5  113.4  122.7  122.3  142.7  214.1  264.7  320.3  389.3  432.9  502.7  155.3  473.8
-//   2 G2 B7    198.5  209.2  221.0  207.5  212.7  214.2  250.2  295.9  351.3  387.2  438.8  241.5  421.7
-//   2 G2 B8    222.7  231.4  243.4  227.6  235.7  234.4  255.3  295.2  349.6  384.8  434.9  264.2  417.3
-//   pooled     276.3  294.2  301.2  272.4  294.2  297.6  304.0  320.0  384.7  421.0  361.9  369.4  456.7
+//   rays         36k    65k    76k    90k   153k   201k   256k   331k   412k   518k   589k  704k   f129k  f518k
+//   8 G3 B6     59.5   78.2   95.4  111.3  167.2  213.0  262.3  332.0  407.1  499.9  561.3  655.6  164.3  577.9
+//   8 G2 B8     60.5   75.8   92.1  107.0  159.8  203.4  250.6  316.6  388.5  476.6  536.5  626.4  156.6  553.2
+//   4 G3 B6     82.4   85.5   88.2   94.7  133.2  168.9  205.9  255.1  310.4  376.9  420.7  490.2  137.1  452.1
+//   4 G2 B8     84.8   89.1   90.5   94.8  128.0  160.4  195.5  241.8  293.7  357.1  398.2  463.4  132.1  429.4
+//   2 G2 B8    145.3  150.6  156.3  152.8  157.7  170.5  184.4  221.2  264.3  316.7  349.2  400.0  184.8  380.7
+//   2 G1 B9    148.2  153.0  159.5  155.4  162.7  174.0  183.1  218.6  260.1  309.5  340.3  389.0  188.6  373.3
+//   pooled     265.9  284.7  279.0  265.6  274.3  282.0  279.5  293.0  299.9  363.8  402.5  335.8  310.2  442.5
+// (8 G6 B4 is 10% slower than 8 G3 B6, 4 G1 B9 within 2% of 4 G2 B8, 10 blocks slower for both.)
 // Launches that run side by side (the views of a batch) fill the GPU together, so their rays together
-// decide: six 512x512 faces and six cameras of 535,000 to 922,000 rays in one call take 2612 us with
-// each view's own choice and 2273 us with half the others' rays counted to its own (batch.cu).  4 G3 stays at 6 blocks though 7 is 3%
-// faster above 150,000 rays: at 7 the compiler contracts other products, and the team sizes would no
-// longer agree to the last bit.  (2 G1 at 8 to 10 blocks, 4 G2 B8, 8 G2 B7 and 8 G3 B5 are slower everywhere or within 1%.)
+// decide, those of the others counted half (batch.cu).
 #ifndef MM_TEAM8_RAYS
-#define MM_TEAM8_RAYS 90000
+#define MM_TEAM8_RAYS 70000
 #endif
 #ifndef MM_TEAM4_RAYS
-#define MM_TEAM4_RAYS 262144
+#define MM_TEAM4_RAYS 240000
 #endif
 #ifndef MM_TEAM2_RAYS
 #define MM_TEAM2_RAYS 600000
@@ -1293,17 +1293,22 @@ struct TeamTile {
 };
 
 // One ray marched by the calling team (member `member` of the kTeam lanes at `base` of the warp; G cone taps
-// issued together).  Every
-// lane of the warp calls it and stays until the last team is done (`inside` = false: a team without a
-// pixel), so the round's results are exchanged by full-warp ballots: three ballots tell every member
-// which samples are valid, hit, and accumulate, and the loop state follows from the bits.  Only a
-// round in which some team of the warp accumulates shuffles values.  Taking the loop body sample by
-// sample on shuffled results instead (up to 16 shuffles under per-team masks a round) made the resolve
-// two fifths of the round: 256x256, teams of 4 with cone taps in sixes at 4 blocks per SM, 147.7 -> 92.8 us.
+// issued together).  Every lane of the warp calls it and stays until the last team is done (`inside` =
+// false: a team without a pixel), so the round's results are exchanged by full-warp ballots: three ballots
+// tell every member which samples are valid, hit, and accumulate, and the loop state follows from the
+// bits; only a round in which some team of the warp accumulates shuffles values.  (The loop body sample by
+// sample on results shuffled under per-team masks, up to 16 shuffles a round: 256x256 147.7 us against
+// 92.8, teams of 4, cone taps in sixes, 4 blocks per SM.)  The sun cones wait in the warp's pool, as in
+// the full-frame kernel: inline, every round with an accumulated sample waited for its cone, three
+// rounds of fetches more for all teams of the warp (256x256 86.7 -> 78.0 us, 1920x1080/16 with the
+// reprojection 152 -> 134).
 template <bool E, int S, bool C, int kTeam, int G>
-__device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, const V3* s_cone, const float& thin,
-                                         int px, int py, bool inside, int member, int base) {
+__device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, const V3* s_cone, ConePool& q,
+                                         const float& thin, int px, int py, bool inside, int member, int base) {
     const unsigned full = 0xffffffffu;
+    const int wp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) q.tail[wp] = 0;
+    int head = 0, pending = 0;  // records of the warp's pool consumed / waiting (the same in every lane)
     Work w;
     Ray r{};
     bool done = true;
@@ -1332,7 +1337,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
             if (member == k) tj = ts[k];
         }
         const bool valid = !done && tj < r.t1 && iterations + member < kMaxIterations;
-        float lo = 0.0f, hi = 0.0f, y = 0.0f;
+        float lo = 0.0f, hi = 0.0f;
         unsigned long long nt = 0, nh = 0;
         if (valid) {
             const V3 pos = f.cam + tj * rd;
@@ -1340,23 +1345,8 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
             F4 cu;
             if (!noHits) cu = curl_fetch<E, S>(p, g);  // issued with the cloudTest fetches
             lo = cloud_test<E, S>(p, f, g, nt);
-            // (teams of 8: a round waits for its slowest lane, so a fetch left out saves nothing and the
-            // test costs 5% of a 256x256 image; teams of 4 and 2 gain 1% and 3%)
-            if (!noHits && lo > 0.0f && (E || kTeam == 8 || lo >= thin || g.rh < 0.1f)) {
+            if (!noHits && lo > 0.0f && (E || lo >= thin || g.rh < 0.1f)) {
                 hi = hires_finish<E>(hires_fetch<E, S>(p, curl_displace<E>(g, stepSize, cu)), g.rh, lo, nh);
-                if (hi >= 0.0001f) {
-                    float dal = 0.0f;
-                    if constexpr (!E) {
-#pragma unroll
-                        for (int i = 0; i < 6; i += G)
-                            dal = cone_taps<E, S, G, true>(p, f, s_cone, i, pos, stepSize, dal, nt, nh);
-                    } else {
-#pragma unroll 1
-                        for (int i = 0; i < 6; i += G)
-                            dal = cone_taps<E, S, G>(p, f, s_cone, i, pos, stepSize, dal, nt, nh);
-                    }
-                    y = shade_term<E>(dal, lo, g.rh, r.cosTheta, r.hg);
-                }
             }
         }
         constexpr unsigned kMask = (1u << kTeam) - 1u;
@@ -1387,10 +1377,11 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
             // ---- the loop body sample by sample on the exchanged results
             const unsigned kb = (kept >> base) & kMask;
             bool run = !done;
+            unsigned pushed = 0;
 #pragma unroll
             for (int i = 0; i < kTeam; ++i) {
                 const float hiv = __shfl_sync(full, hi, base + i);
-                const float yi = __shfl_sync(full, y, base + i);
+                const float loi = __shfl_sync(full, lo, base + i);
                 unsigned ti = 0, hn = 0;
                 if (C) {
                     ti = __shfl_sync(full, (unsigned)nt, base + i);
@@ -1402,7 +1393,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                 }
                 if (run) {
                     ++used;
-                    if (C) {
+                    if (C && member == 0) {
                         ++w.iter;
                         w.test += ti;
                         w.hires += hn;
@@ -1413,8 +1404,17 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                         if (noHits) {  // :428-434
                             turn = true;
                         } else if ((kb >> i) & 1u) {  // :437-466
-                            transmittance = mixf(transmittance, yi, 1.0f - accum);
-                            if (C) ++w.acc;
+                            // its cone and blend (:441-462) come later, in the pool's order
+                            if (member == 0) {
+                                const int slot = atomicAdd(&q.tail[wp], 1) & (kPool - 1);
+                                q.t[wp][slot] = ts[i];
+                                q.step[wp][slot] = stepSize;
+                                q.lm[wp][slot].lo = loi;
+                                q.acc[wp][slot] = accum;
+                                q.own[wp][slot] = (unsigned char)(base);
+                                if (C) ++w.acc;
+                                ++pushed;
+                            }
                             if (firstT == CUDART_INF_F) firstT = ts[i];
                             accum += hiv;
                             count = true;
@@ -1435,6 +1435,12 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                     run = !(done || turn || back);
                 }
             }
+            pending += (int)__reduce_add_sync(full, pushed);
+            if (pending >= 32) {  // at most 32 appended a round
+                cone_round<E, S, G>(p, f, s_cone, q, head, 32, rd, transmittance, r.cosTheta, r.hg, w);
+                head += 32;
+                pending -= 32;
+            }
         }
         // ---- on to the next round: the increment (:408), after a step back half a step (:428-434)
         // or a return to large steps
@@ -1454,10 +1460,10 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
         }
         t += stepSize;
     }
-    if (live && member == 0) {
+    if (pending > 0) cone_round<E, S, G>(p, f, s_cone, q, head, pending, rd, transmittance, r.cosTheta, r.hg, w);
+    if (live && member == 0)
         store_pixel(p, px, py, composite<E>(p.u, f, r.rd, r.bg, r.alpha, accum, transmittance), firstT);
-        if (C) flush_work(p.counters, w);
-    }
+    if (C) flush_work(p.counters, w);
 }
 
 // One launch: the first team_blocks blocks march the ray rows above the horizon by teams, from the
@@ -1472,6 +1478,7 @@ struct TeamGrid {
 template <bool E, int S, bool C, int kTeam, int G, int kMinBlocks>
 __global__ void __launch_bounds__(128, kMinBlocks) march_team_kernel(MarchLaunch p, TeamGrid tg) {
     __shared__ V3 s_cone[6];
+    __shared__ ConePool s_q;
     __shared__ float s_thin;
     cone_offsets(p.u, s_cone);
     if (!E && threadIdx.x == 0) s_thin = thin_density(p);
@@ -1501,7 +1508,7 @@ __global__ void __launch_bounds__(128, kMinBlocks) march_team_kernel(MarchLaunch
     const bool inside = px < p.width && py < p.height;
     const Frame f = make_frame<E>(p);
     if (team_block) {  // every lane of the warp stays: the rounds' ballots need them all
-        team_ray<E, S, C, kTeam, G>(p, f, s_cone, s_thin, px, py, inside, lane % kTeam, lane / kTeam * kTeam);
+        team_ray<E, S, C, kTeam, G>(p, f, s_cone, s_q, s_thin, px, py, inside, lane % kTeam, lane / kTeam * kTeam);
     } else if (inside) {
         Work w;
         march_pixel<E, S>(p, f, s_cone, px, py, w);
@@ -1637,11 +1644,11 @@ int launch_tiled(const MarchLaunch& p0, cudaStream_t s, bool half2 = false, long
     const bool h2 = !E && S == MM_SAMPLER_HARDWARE && half2 && p.pixel_mode != MM_PIXELS_PHASE16;
     if (rays <= (h2 ? kHalf2Rays : kTeam2Rays)) {
         if (rays <= kTeam8Rays)
-            launch_team<E, S, 8, E ? 1 : 3, E ? 3 : 6>(p, gw, gh, s);
+            launch_team<E, S, 8, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
         else if (rays <= kTeam4Rays)
-            launch_team<E, S, 4, E ? 1 : 3, E ? 3 : 6>(p, gw, gh, s);
+            launch_team<E, S, 4, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
         else
-            launch_team<E, S, 2, E ? 1 : 2, E ? 3 : 7>(p, gw, gh, s);
+            launch_team<E, S, 2, 1, E ? 4 : 9>(p, gw, gh, s);
     } else if (h2) {
         if constexpr (!E && S == MM_SAMPLER_HARDWARE) {
             if (C)

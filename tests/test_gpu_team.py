@@ -6,7 +6,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # rays just below and above each line of the dispatch, odd sides; a small image; the pooled kernel's first
-SIZES = [(5, 3), (301, 299), (301, 300), (509, 513), (517, 509), (775, 773), (777, 773)]
+SIZES = [(5, 3), (263, 266), (301, 299), (301, 300), (479, 501), (481, 500), (509, 513), (517, 509), (775, 773),
+         (777, 773)]
 
 
 @pytest.fixture(scope="module")
