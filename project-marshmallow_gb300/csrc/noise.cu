@@ -175,13 +175,14 @@ __device__ float value2(float qx, float qy, int f, uint32_t s) {
 // lane a column of kRun texels): one unit per Worley channel and, for the low-res volume, one for the
 // Perlin octaves.  For each octave a unit first hashes the cells its tile can reach into shared memory,
 // once per cell instead of 27 times per texel, then every lane takes its 27 neighbours from there.  The
-// texels of a column that lie in the same cell along z (4 at a time, 2, or 1: the same for every lane) go
+// texels of a column that lie in the same cell along z (8 at a time, 4, 2, or 1: the same for every lane) go
 // through a neighbour together: its x and y distances are theirs in common, which leaves a subtraction,
 // a product, a sum and a minimum each.  Every float operation is worley3's own, so the texels are the same
 // bytes.  Where an octave has more cells in reach than the table holds (more than about half a cell per
 // texel), its texels are computed one by one as before.
 // Bound by FP32 issue: 27 distances x 12 octaves a texel.  us at the start -> with the tables -> with packed FP32
-// operations: low-res 128^3 1229 -> 226 -> 201, 64^3 164 -> 56 -> 52; hi-res 32^3 27 -> 11, 64^3 109 -> 27 -> 25.
+// operations -> 8 texels at a time: low-res 128^3 1229 -> 226 -> 201 -> 183, 64^3 164 -> 56 -> 52; hi-res 32^3
+// 27 -> 11, 64^3 109 -> 27 -> 25 -> 23.
 // (Passing over rows of cells no closer than the distance found so far costs what it saves: 232 -> 240.)
 constexpr int kCells = 680;         // table entries of a Worley unit: 32 x 2 x 8 texels at 0.55 cells a texel
 constexpr int kPerlinCells = 256;   // of the Perlin unit, whose octaves are the coarse ones
@@ -345,11 +346,22 @@ __global__ void __launch_bounds__(320) volume_kernel(int kind, uint32_t seed, in
                 s_sum[r][threadIdx.x] = o ? s_sum[r][threadIdx.x] + w : w;
             };
 #pragma unroll 1
-            for (int r = 0; r < kRun;) {  // the next 4, 2 or 1 texels of the column that share a cell
+            for (int r = 0; r < kRun;) {  // the next 8, 4, 2 or 1 texels of the column that share a cell
                 const int c = __shfl_sync(full, cl, r);
                 const bool two = r + 1 < kRun && __shfl_sync(full, cl, r + 1) == c;
                 const bool four = r + 3 < kRun && __shfl_sync(full, cl, r + 3) == c;
                 const float* at = column + (c - 1 - z0) * nxy;
+                if constexpr (kRun == 8) {
+                    if (r == 0 && __shfl_sync(full, cl, 7) == c) {
+                        float fz[8], best[8];
+#pragma unroll
+                        for (int m = 0; m < 8; ++m) fz[m] = __shfl_sync(full, fl, m);
+                        nearest<8>(at, kCells, nx, nxy, fx, fy, fz, best);
+#pragma unroll
+                        for (int m = 0; m < 8; ++m) add(m, best[m]);
+                        break;
+                    }
+                }
                 float fz[4], best[4];
 #pragma unroll
                 for (int m = 0; m < 4; ++m) fz[m] = __shfl_sync(full, fl, r + m);
