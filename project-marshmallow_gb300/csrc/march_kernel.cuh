@@ -24,14 +24,17 @@
 // Build knobs (defaults measured best on GB300 at 3840x2160): warps per block of the tiled kernels
 // (4 or 8) and the minimum resident blocks per SM requested from the register allocator for them
 // (4 warps x 10 blocks: 48 registers, 40 warps per SM; the inline-cone kernel has no spills there and
-// was 4.6% slower at 9 blocks / 56 registers; the pooled-cone kernel spills 64 B in its cone rounds
-// and was 2.6% / 5.1% slower at 9 / 11 blocks); the same for the persistent kernel; and the
+// was 4.6% slower at 9 blocks / 56 registers), for the pooled-cone kernel (12 blocks: march_pixel_q) and
+// for the persistent kernel; and the
 // speculative curl fetch of the tiled march (off: it costs more occupancy than it hides).
 #ifndef MM_TILED_WARPS
 #define MM_TILED_WARPS 4
 #endif
 #ifndef MM_MARCH_MIN_BLOCKS
 #define MM_MARCH_MIN_BLOCKS (MM_TILED_WARPS == 4 ? 10 : 5)
+#endif
+#ifndef MM_POOL_MIN_BLOCKS
+#define MM_POOL_MIN_BLOCKS (MM_TILED_WARPS == 4 ? 12 : 6)
 #endif
 #ifndef MM_PERSISTENT_MIN_BLOCKS
 #define MM_PERSISTENT_MIN_BLOCKS 3
@@ -1008,7 +1011,8 @@ __device__ __forceinline__ void march_tiled_body(const MarchLaunch& p) {
 // the per-iteration count became one reduction).  Every sample, tap and blend is the shader's
 // arithmetic in its order per ray, so results and work counts equal the one-thread march bit for bit
 // in exact mode.
-constexpr int kPool = 64;  // records per warp: < 32 after a round, + at most 32 per iteration
+constexpr int kPool = 63;  // records per warp: < 32 after a round, + at most 32 per iteration
+__device__ __forceinline__ int pool_slot(int i) { return i < kPool ? i : i - kPool; }  // i < 2 kPool
 // Cone taps a lane of a round issues together (1, 2, 3 or 6).  3840x2160 / 1920x1080 sweeps: one at
 // a time 3.215 / 0.992 ms; in pairs 3.347 / 1.036 (spills at 48 registers), 3.328 / 1.025 at 9 blocks
 // per SM; in threes 3.819 / 1.186.
@@ -1028,8 +1032,11 @@ struct ConePool {
         unsigned mask;  // during a round, at slot head + o: the round's lanes holding owner o's records
     } lm[MM_TILED_WARPS][kPool];
     unsigned char own[MM_TILED_WARPS][kPool];
-    int tail[MM_TILED_WARPS];  // records appended so far (slot = index mod kPool)
+    int waiting[MM_TILED_WARPS];  // records behind the pool's head
+    float thin;                   // thin_density, for the block
 };
+// 12 blocks of the pooled kernel, 1 KB reserved for each, fill a 64 KB carveout.
+static_assert(MM_TILED_WARPS != 4 || sizeof(ConePool) <= 4352, "pool size");
 
 // One round: the `take` (<= 32) oldest records of the warp's pool, one per lane, then each owner's
 // blends in pool order.  Every lane of the warp calls it with the same head and take.
@@ -1042,7 +1049,7 @@ __device__ __forceinline__ void cone_round(const MarchLaunch& p, const Frame& f,
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     __syncwarp();  // the appended records are visible to the warp
     const bool work = lane < take;
-    const int slot = (head + lane) & (kPool - 1);
+    const int slot = pool_slot(head + lane);
     const int o = work ? (int)q.own[wp][slot] : 32 + lane;  // idle lanes: a value no owner has
     const int src = o & 31;
     const float rx = __shfl_sync(full, rd.x, src), ry = __shfl_sync(full, rd.y, src);
@@ -1067,124 +1074,130 @@ __device__ __forceinline__ void cone_round(const MarchLaunch& p, const Frame& f,
     q.lm[wp][slot].mask = 0u;  // this lane's slot of the round: read above (if it held a record)
     const unsigned same = __match_any_sync(full, o);
     __syncwarp();
-    if (work && lane == __ffs(same) - 1) q.lm[wp][(head + o) & (kPool - 1)].mask = same;
+    if (work && lane == __ffs(same) - 1) q.lm[wp][pool_slot(head + o)].mask = same;
     __syncwarp();
     unsigned mine = q.lm[wp][slot].mask;
     while (mine) {  // :462, in accumulation order
-        const int sl = (head + __ffs(mine) - 1) & (kPool - 1);
+        const int sl = pool_slot(head + __ffs(mine) - 1);
         mine &= mine - 1u;
         trans = mixf(trans, q.t[wp][sl], 1.0f - q.acc[wp][sl]);
     }
+    if (lane == 0) q.waiting[wp] -= take;
     __syncwarp();  // the round's slots are read before later appends reuse them
 }
 
 // The march of pixel (px, py) with deferred sun cones (inside = false: no pixel, a helper lane).
 template <bool E, int S, bool SC>
 __device__ __forceinline__ void march_pixel_q(const MarchLaunch& p, const Frame& f, const V3* cone, ConePool& q,
-                                              const float& thin, int px, int py, bool inside, Work& w) {
+                                              int px, int py, bool inside, Work& w) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     Ray r{};
     bool live = false;
     if (inside) {
         r = ray_setup<E, S>(p, f, px, py);
-        if (r.killed)
-            store_pixel(p, px, py, make_float4(r.bg.x, r.bg.y, r.bg.z, r.alpha), CUDART_INF_F);
-        else
-            live = true;
+        live = !r.killed;
+        // The background waits in the image: four registers less through the march, which with a pool of
+        // 63 records (12 blocks in the 64 KB carveout) lets 12 blocks of 40 registers pay: 3840x2160 2759 ->
+        // 2705 us, 1920x1080 789 -> 779 (10 blocks of 48: 2759 / 790; a 100 KB carveout 2712 / 781).
+        store_pixel(p, px, py, make_float4(r.bg.x, r.bg.y, r.bg.z, r.alpha), CUDART_INF_F);
     }
-    if (lane == 0) q.tail[wp] = 0;
+    if (lane == 0) q.waiting[wp] = 0;
     float accum = 0.0f, trans = 1.0f;
     float stepSize = 0.05f * f.thickness;  // :390
     bool noHits = true;
-    int misses = 0, steps = 0, iterations = 0;
+    int misses = 0, steps = 0;
     int head = 0, pending = 0;  // records of the warp's pool consumed / waiting (the same in every lane)
     float firstT = CUDART_INF_F;
     float t = r.t0;
     bool alive = live && t < r.t1;  // :408, the loop condition on entry
     __syncwarp();
-    for (;;) {
+    // A trip is one iteration of every ray still marching, so its number is the rays' iteration count.
+    // Issue bounds the loop (80% of the slots, 748 M warp instructions at 1920x1080), so a trip does no
+    // more than it must: the opacity is looked at where it changes, and two votes tell whether anything
+    // was appended (one trip in twelve) and whether any ray goes on: 3840x2160 2775 -> 2759 us, 1920x1080 797
+    // -> 789, 16 bytes of spills instead of 64.  (Records written behind the vote, at the lane's rank in it,
+    // instead of behind an atomic where they arise: 2759 -> 2820.)
+    for (int trip = 0;; ++trip) {
         bool pushed = false;
         if (alive) {  // one iteration of :408-482
             ++w.iter;
-            bool next = true;  // false: the loop ends here (no increment)
+            bool counted = true;  // false: the shader's `continue`
             const V3 pos = f.cam + t * r.rd;
             const Geo g = geo_at<E>(f, pos);
             F4 cu;
             if (SC && !noHits) cu = curl_fetch<E, S>(p, g);
             float density = cloud_test<E, S>(p, f, g, w.test);
             const float loDensity = density;
-            do {  // `break` = the shader's `continue`
-                if (density > 0.0f) {
-                    misses = 0;
-                    if (noHits) {  // :428-434
-                        t -= stepSize;
-                        stepSize *= 0.3f;
-                        noHits = false;
-                        break;
-                    }
-                    if (!E && density < thin && g.rh >= 0.1f) break;  // eroded away (thin_density)
+            if (density > 0.0f) {
+                misses = 0;
+                counted = false;
+                if (noHits) {  // :428-434
+                    t -= stepSize;
+                    stepSize *= 0.3f;
+                    noHits = false;
+                } else if (E || density >= q.thin || g.rh < 0.1f) {  // else eroded away (thin_density)
                     if (SC)
                         density = hires_finish<E>(hires_fetch<E, S>(p, curl_displace<E>(g, stepSize, cu)), g.rh,
                                                   density, w.hires);
                     else
                         density = cloud_hires<E, S>(p, g, stepSize, density, w.hires);
-                    if (density < 0.0001f) break;
-                    // the cone and blend of this sample (:441-462) come later; an owner's records
-                    // take increasing slots, so the pool keeps each ray's order
-                    const int slot = atomicAdd(&q.tail[wp], 1) & (kPool - 1);
-                    q.t[wp][slot] = t;
-                    q.step[wp][slot] = stepSize;
-                    q.lm[wp][slot].lo = loDensity;
-                    q.acc[wp][slot] = accum;
-                    q.own[wp][slot] = (unsigned char)lane;
-                    pushed = true;
-                    ++w.acc;
-                    if (firstT == CUDART_INF_F) firstT = t;
-                    accum += density;
-                } else if (!noHits) {  // :468-474
-                    misses++;
-                    if (misses >= 10) {
-                        noHits = true;
-                        stepSize = M<E>::div(stepSize, 0.3f);
+                    if (density >= 0.0001f) {
+                        // the cone and blend of this sample (:441-462) come later; an owner's records
+                        // take increasing slots, so the pool keeps each ray's order
+                        const int slot = pool_slot(head + atomicAdd(&q.waiting[wp], 1));
+                        q.t[wp][slot] = t;
+                        q.step[wp][slot] = stepSize;
+                        q.lm[wp][slot].lo = loDensity;
+                        q.acc[wp][slot] = accum;
+                        q.own[wp][slot] = (unsigned char)lane;
+                        pushed = true;
+                        ++w.acc;
+                        if (firstT == CUDART_INF_F) firstT = t;
+                        accum += density;
+                        if (accum > 0.99f) {  // :476-479
+                            accum = 1.0f;
+                            alive = false;
+                        } else {
+                            counted = true;
+                        }
                     }
                 }
-                if (accum > 0.99f) {
-                    accum = 1.0f;
-                    next = false;
-                    break;
+            } else if (!noHits) {  // :468-474
+                misses++;
+                if (misses >= 10) {
+                    noHits = true;
+                    stepSize = M<E>::div(stepSize, 0.3f);
                 }
-                if (++steps > 100) next = false;
-            } while (false);
-            if (next) {
-                t += stepSize;
-                ++iterations;
-                alive = t < r.t1 && iterations < kMaxIterations;
-            } else {
-                alive = false;
+            }
+            if (counted && ++steps > 100) alive = false;  // :481
+            t += stepSize;
+            alive = alive && t < r.t1;
+        }
+        const unsigned appended = __ballot_sync(full, pushed);
+        if (appended) {
+            pending += __popc(appended);
+            if (pending >= 32) {  // < 64 records: < 32 after a round, at most 32 appended since
+                cone_round<E, S, MM_POOL_CONE_GROUP>(p, f, cone, q, head, 32, r.rd, trans, r.cosTheta, r.hg, w);
+                head = pool_slot(head + 32);
+                pending -= 32;
             }
         }
-        // one reduction gives the records appended (low 6 bits) and the rays still marching (x 64)
-        const unsigned sum = __reduce_add_sync(full, (pushed ? 1u : 0u) + (alive ? 64u : 0u));
-        pending += (int)(sum & 63u);
-        if (pending >= 32) {  // < 64 records: < 32 after a round, at most 32 appended since
-            cone_round<E, S, MM_POOL_CONE_GROUP>(p, f, cone, q, head, 32, r.rd, trans, r.cosTheta, r.hg, w);
-            head += 32;
-            pending -= 32;
-        }
-        if (sum < 64u) break;
+        if (!__any_sync(full, alive) || trip + 1 >= kMaxIterations) break;
     }
     if (pending > 0) cone_round<E, S, MM_POOL_CONE_GROUP>(p, f, cone, q, head, pending, r.rd, trans, r.cosTheta, r.hg, w);
-    if (live) store_pixel(p, px, py, composite<E>(p.u, f, r.rd, r.bg, r.alpha, accum, trans), firstT);
+    if (live) {
+        const float4 b = *(reinterpret_cast<const float4*>(reinterpret_cast<const char*>(p.rgba) + (size_t)py * p.rgba_pitch) + px);
+        store_pixel(p, px, py, composite<E>(p.u, f, r.rd, V3{b.x, b.y, b.z}, b.w, accum, trans), firstT);
+    }
 }
 
 template <bool E, int S, bool C, bool SC>
 __device__ __forceinline__ void march_tiled_q_body(const MarchLaunch& p) {
     __shared__ V3 s_cone[6];
     __shared__ ConePool s_q;
-    __shared__ float s_thin;
     cone_offsets(p.u, s_cone);
-    if (!E && threadIdx.x == 0) s_thin = thin_density(p);
+    if (!E && threadIdx.x == 0) s_q.thin = thin_density(p);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int by = (int)blockIdx.y < p.row_split ? p.row_split - 1 - (int)blockIdx.y : (int)blockIdx.y;
@@ -1197,7 +1210,7 @@ __device__ __forceinline__ void march_tiled_q_body(const MarchLaunch& p) {
     }
     const Frame f = make_frame<E>(p);
     Work w;
-    march_pixel_q<E, S, SC>(p, f, s_cone, s_q, s_thin, px, py, px < p.width && py < p.height, w);
+    march_pixel_q<E, S, SC>(p, f, s_cone, s_q, px, py, px < p.width && py < p.height, w);
     if (C) flush_work(p.counters, w);
 }
 
@@ -1228,7 +1241,7 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_MARCH_MIN_BLOCKS) marc
 
 // Full frames with deferred, pooled sun cones (above).
 template <bool E, int S, bool C>
-__global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_MARCH_MIN_BLOCKS) march_tiled_pool_kernel(MarchLaunch p) {
+__global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_POOL_MIN_BLOCKS) march_tiled_pool_kernel(MarchLaunch p) {
     march_tiled_q_body<E, S, C, (MM_SPEC_CURL != 0)>(p);
 }
 
@@ -1304,10 +1317,10 @@ struct TeamTile {
 // reprojection 152 -> 134).
 template <bool E, int S, bool C, int kTeam, int G>
 __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, const V3* s_cone, ConePool& q,
-                                         const float& thin, int px, int py, bool inside, int member, int base) {
+                                         int px, int py, bool inside, int member, int base) {
     const unsigned full = 0xffffffffu;
     const int wp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) q.tail[wp] = 0;
+    if ((threadIdx.x & 31) == 0) q.waiting[wp] = 0;
     int head = 0, pending = 0;  // records of the warp's pool consumed / waiting (the same in every lane)
     Work w;
     Ray r{};
@@ -1345,7 +1358,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
             F4 cu;
             if (!noHits) cu = curl_fetch<E, S>(p, g);  // issued with the cloudTest fetches
             lo = cloud_test<E, S>(p, f, g, nt);
-            if (!noHits && lo > 0.0f && (E || lo >= thin || g.rh < 0.1f)) {
+            if (!noHits && lo > 0.0f && (E || lo >= q.thin || g.rh < 0.1f)) {
                 hi = hires_finish<E>(hires_fetch<E, S>(p, curl_displace<E>(g, stepSize, cu)), g.rh, lo, nh);
             }
         }
@@ -1406,7 +1419,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                         } else if ((kb >> i) & 1u) {  // :437-466
                             // its cone and blend (:441-462) come later, in the pool's order
                             if (member == 0) {
-                                const int slot = atomicAdd(&q.tail[wp], 1) & (kPool - 1);
+                                const int slot = pool_slot(head + atomicAdd(&q.waiting[wp], 1));
                                 q.t[wp][slot] = ts[i];
                                 q.step[wp][slot] = stepSize;
                                 q.lm[wp][slot].lo = loi;
@@ -1438,7 +1451,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
             pending += (int)__reduce_add_sync(full, pushed);
             if (pending >= 32) {  // at most 32 appended a round
                 cone_round<E, S, G>(p, f, s_cone, q, head, 32, rd, transmittance, r.cosTheta, r.hg, w);
-                head += 32;
+                head = pool_slot(head + 32);
                 pending -= 32;
             }
         }
@@ -1479,9 +1492,8 @@ template <bool E, int S, bool C, int kTeam, int G, int kMinBlocks>
 __global__ void __launch_bounds__(128, kMinBlocks) march_team_kernel(MarchLaunch p, TeamGrid tg) {
     __shared__ V3 s_cone[6];
     __shared__ ConePool s_q;
-    __shared__ float s_thin;
     cone_offsets(p.u, s_cone);
-    if (!E && threadIdx.x == 0) s_thin = thin_density(p);
+    if (!E && threadIdx.x == 0) s_q.thin = thin_density(p);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int tx, ty;
@@ -1508,7 +1520,7 @@ __global__ void __launch_bounds__(128, kMinBlocks) march_team_kernel(MarchLaunch
     const bool inside = px < p.width && py < p.height;
     const Frame f = make_frame<E>(p);
     if (team_block) {  // every lane of the warp stays: the rounds' ballots need them all
-        team_ray<E, S, C, kTeam, G>(p, f, s_cone, s_q, s_thin, px, py, inside, lane % kTeam, lane / kTeam * kTeam);
+        team_ray<E, S, C, kTeam, G>(p, f, s_cone, s_q, px, py, inside, lane % kTeam, lane / kTeam * kTeam);
     } else if (inside) {
         Work w;
         march_pixel<E, S>(p, f, s_cone, px, py, w);
@@ -1577,14 +1589,13 @@ inline int horizon_row_split(const MarchLaunch& p, int block_rows, int rows_per_
 // 16-frame sweep, 60 degree field of view, inline -> pooled: 1920x1080 1.074 -> 0.993 ms, 2880x1620
 // 1.988 -> 1.924, 3200x1800 2.394 -> 2.338, 3840x2160 3.240 -> 3.212.
 
-// The pooled kernel's shared memory is small (4.4 KB a block), and the rest of the SM's unified L1 is
-// its texture cache.  Without a preference the driver gave it a 132 KB shared-memory carveout; the
-// preference computed from its need (10 blocks x (4.4 + 1 KB reserved) = 23% of 228 KB) still got
-// 100 KB, and 20% (or 12%) got 64 KB, which holds 11 blocks (6%: 32 KB, 5 blocks).  1920x1080, one
-// sweep frame: L1 hit rate 88% / 91.4% / 93.0% at 132 / 100 / 64 KB (the inline kernel: 93.0% at its
-// 32 KB); 16-frame sweep at 64 KB against 100 KB: 1920x1080 1.012 / 1.021 ms, 3840x2160 3.273 /
-// 3.295.  So 20% is requested (MM_POOL_CARVEOUT_PCT = 0: the computed preference) when a context is
-// created, outside any stream capture.  A hint only: a failure is cleared and ignored.
+// The pooled kernel's shared memory is small (4.3 KB a block), and the rest of the SM's unified L1 is its
+// texture cache.  Without a preference the driver gave it a 132 KB shared-memory carveout; 20% (or 12%)
+// gets 64 KB, which holds 12 blocks with the 1 KB reserved for each, 25% and 30% get 100 KB, 6% 32 KB (5
+// blocks).  3840x2160 / 1920x1080 at 64 KB against 100 KB: 2705 / 779 us against 2712 / 781 (L1 hit rates with
+// 10 blocks: 93.0% at 64 KB, 91.4% at 100, 88% at 132).  So 20% is requested (MM_POOL_CARVEOUT_PCT = 0: the
+// computed preference) when a context is created, outside any stream capture.  A hint only: a failure is
+// cleared and ignored.
 template <bool E, int S, bool C>
 void pool_carveout() {
     if (!MM_MARCH_CARVEOUT) return;
@@ -1598,7 +1609,7 @@ void pool_carveout() {
     if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess &&
         cudaFuncGetAttributes(&a, march_tiled_pool_kernel<E, S, C>) == cudaSuccess && per_sm > 0) {
-        const long long need = (long long)MM_MARCH_MIN_BLOCKS * ((long long)a.sharedSizeBytes + reserved);
+        const long long need = (long long)MM_POOL_MIN_BLOCKS * ((long long)a.sharedSizeBytes + reserved);
         int pct = MM_POOL_CARVEOUT_PCT > 0 ? MM_POOL_CARVEOUT_PCT : (int)((100 * need + per_sm - 1) / per_sm);
         pct = pct < 1 ? 1 : (pct > 100 ? 100 : pct);
         cudaFuncSetAttribute(march_tiled_pool_kernel<E, S, C>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
