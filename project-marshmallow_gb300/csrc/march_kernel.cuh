@@ -1341,13 +1341,11 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
     float t = r.t0;
     while (__any_sync(full, !done)) {
         // ---- the round's positions (the loop's own additions) and this member's sample
-        float ts[kTeam];
-        ts[0] = t;
-        float tj = t;
+        float tj = t, tk = t;
 #pragma unroll
         for (int k = 1; k < kTeam; ++k) {
-            ts[k] = ts[k - 1] + stepSize;
-            if (member == k) tj = ts[k];
+            tk += stepSize;
+            if (member == k) tj = tk;
         }
         const bool valid = !done && tj < r.t1 && iterations + member < kMaxIterations;
         float lo = 0.0f, hi = 0.0f;
@@ -1391,13 +1389,15 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
             const unsigned kb = (kept >> base) & kMask;
             bool run = !done;
             unsigned pushed = 0;
-#pragma unroll
-            for (int i = 0; i < kTeam; ++i) {
+            float ti = t;  // position of sample i
+            constexpr int kUnroll = kTeam == 8 ? 1 : kTeam;  // (8 times over, instruction fetches stall it)
+#pragma unroll kUnroll
+            for (int i = 0; i < kTeam; ++i, ti += stepSize) {
                 const float hiv = __shfl_sync(full, hi, base + i);
                 const float loi = __shfl_sync(full, lo, base + i);
-                unsigned ti = 0, hn = 0;
+                unsigned tn = 0, hn = 0;
                 if (C) {
-                    ti = __shfl_sync(full, (unsigned)nt, base + i);
+                    tn = __shfl_sync(full, (unsigned)nt, base + i);
                     hn = __shfl_sync(full, (unsigned)nh, base + i);
                 }
                 if (run && !((vb >> i) & 1u)) {  // the loop condition fails: the ray is finished
@@ -1408,7 +1408,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                     ++used;
                     if (C && member == 0) {
                         ++w.iter;
-                        w.test += ti;
+                        w.test += tn;
                         w.hires += hn;
                     }
                     bool count = false;
@@ -1420,7 +1420,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                             // its cone and blend (:441-462) come later, in the pool's order
                             if (member == 0) {
                                 const int slot = pool_slot(head + atomicAdd(&q.waiting[wp], 1));
-                                q.t[wp][slot] = ts[i];
+                                q.t[wp][slot] = ti;
                                 q.step[wp][slot] = stepSize;
                                 q.lm[wp][slot].lo = loi;
                                 q.acc[wp][slot] = accum;
@@ -1428,7 +1428,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                                 if (C) ++w.acc;
                                 ++pushed;
                             }
-                            if (firstT == CUDART_INF_F) firstT = ts[i];
+                            if (firstT == CUDART_INF_F) firstT = ti;
                             accum += hiv;
                             count = true;
                         }
@@ -1458,9 +1458,14 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
         // ---- on to the next round: the increment (:408), after a step back half a step (:428-434)
         // or a return to large steps
         iterations += used;
+        if constexpr (kTeam == 8) {
+            const float last = __shfl_sync(full, tj, base + (used ? used - 1 : 0));
+            if (used) t = last;
+        } else {
 #pragma unroll
-        for (int k = 0; k < kTeam; ++k)
-            if (used == k + 1) t = ts[k];
+            for (int k = 1; k < kTeam; ++k)
+                if (used > k) t += stepSize;
+        }
         if (turn) {
             misses = 0;
             t -= stepSize;
