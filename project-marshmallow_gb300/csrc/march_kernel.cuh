@@ -1269,32 +1269,59 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PAIR_MIN_BLOCKS) march
 //
 // Which launches take teams, and of how many lanes.  A launch takes at least as long as its longest
 // rays, ~300 us one thread per ray; a team of n lanes makes that chain shorter, but costs lanes: each
-// member sets the ray up, and a round's tail is dropped at every step-size change.  The more rays, the
-// smaller the teams; past ~600,000 rays the pooled kernel's throughput wins.  Cone taps in groups of G
-// at B blocks per SM: a larger G shortens a cone round, a larger B helps the launch.  Microseconds on GB300,
-// pitch 12, two seeds, whole images and (f) frames with 1 pixel in 16 marched (the reprojection beside):
-//   rays         36k    65k    76k    90k   153k   201k   256k   331k   412k   518k   589k  704k   f129k  f518k
-//   8 G3 B6     59.5   78.2   95.4  111.3  167.2  213.0  262.3  332.0  407.1  499.9  561.3  655.6  164.3  577.9
-//   8 G2 B8     60.5   75.8   92.1  107.0  159.8  203.4  250.6  316.6  388.5  476.6  536.5  626.4  156.6  553.2
-//   4 G3 B6     82.4   85.5   88.2   94.7  133.2  168.9  205.9  255.1  310.4  376.9  420.7  490.2  137.1  452.1
-//   4 G2 B8     84.8   89.1   90.5   94.8  128.0  160.4  195.5  241.8  293.7  357.1  398.2  463.4  132.1  429.4
-//   2 G2 B8    145.3  150.6  156.3  152.8  157.7  170.5  184.4  221.2  264.3  316.7  349.2  400.0  184.8  380.7
-//   2 G1 B9    148.2  153.0  159.5  155.4  162.7  174.0  183.1  218.6  260.1  309.5  340.3  389.0  188.6  373.3
-//   pooled     265.9  284.7  279.0  265.6  274.3  282.0  279.5  293.0  299.9  363.8  402.5  335.8  310.2  442.5
-// (8 G6 B4 is 10% slower than 8 G3 B6, 4 G1 B9 within 2% of 4 G2 B8, 10 blocks slower for both.)
+// member sets the ray up, and a round's tail is dropped at every step-size change.  So what decides is the
+// launch's work in units of its longest rays: its rays times the mean length of a ray inside the cloud shell
+// over the longest one (crowding: 0.36 for 960x540 at 60 degrees pitched up by 12, 0.25 from 8 km up, 0.8 at
+// 8 degrees pitched up by 3).  The more of it, the smaller the teams; in the end the pooled kernel's throughput
+// wins.  Cone taps in groups of G at B blocks per SM: 8 G2 B8, 4 G2 B8, 2 G1 B9 (8 G3 B6 is 3% slower at its
+// line, 8 G6 B4 10%, 10 blocks slower for 4 and 2).  Microseconds on GB300 around the lines, whole images,
+// "view, size (work in thousands)"; @15: 15 degrees wide, pitched up by 20:
+//                               8      4                                4      2                              2   pooled
+//   pitch 25, 256x256 (25.3)   90.2  105.7   down 20, 960x540 (86)   182.0  193.7   pitch 12, 960x540 (185) 325.8  378.7
+//   level, 400x225 (27.3)      91.2  105.4   pitch 12, 512x512 (90)  196.5  191.2   pitch 25, 800x600 (188) 340.0  358.1
+//   pitch 5, 400x225 (28.5)    97.6  103.8   @15, 480x270 (97)       142.2  134.9   @15, 512x512 (197)      215.0  178.9
+//   pitch 12, 400x225 (32.0)  106.7   98.9   8 km, 640x640 (101)     256.1  226.7   pitch 25, 960x540 (207) 374.9  406.5
+//   8 km, 480x270 (32.3)      123.1  111.2   pitch 25, 512x512 (101) 225.8  200.4   pitch 5, 960x720 (215)  359.5  353.2
+//   pitch 25, 400x225 (36.0)  122.8  107.6   level, 640x640 (120)    239.4  217.7   pitch 12, 960x720 (240) 395.1  372.7
+// Over 72 such views the lines below take the best of the four or one within 20% of it; lines by the number
+// of rays alone are up to 57% off it.
 // Launches that run side by side (the views of a batch) fill the GPU together, so their rays together
-// decide, those of the others counted half (batch.cu).
-#ifndef MM_TEAM8_RAYS
-#define MM_TEAM8_RAYS 70000
+// decide, those of the others counted half (batch.cu), all at a 60 degree camera's crowding (each view at its
+// own: four batches of small cube maps and cameras 278, 464, 350 and 315 us for 268, 422, 319 and 315).
+#ifndef MM_TEAM8_WORK
+#define MM_TEAM8_WORK 30000
 #endif
-#ifndef MM_TEAM4_RAYS
-#define MM_TEAM4_RAYS 240000
+#ifndef MM_TEAM4_WORK
+#define MM_TEAM4_WORK 90000
 #endif
-#ifndef MM_TEAM2_RAYS
-#define MM_TEAM2_RAYS 600000
+#ifndef MM_TEAM2_WORK
+#define MM_TEAM2_WORK 212000
 #endif
-constexpr long long kTeam8Rays = MM_TEAM8_RAYS, kTeam4Rays = MM_TEAM4_RAYS, kTeam2Rays = MM_TEAM2_RAYS;
-constexpr long long kHalf2Rays = 262144;  // MM_MATH_FAST_HALF2: images up to here take teams (FP32 decisions)
+constexpr double kCrowdingBeside = 0.37;
+constexpr double kTeam8Work = MM_TEAM8_WORK, kTeam4Work = MM_TEAM4_WORK, kTeam2Work = MM_TEAM2_WORK;
+constexpr long long kHalf2Rays = 262144;  // MM_MATH_FAST_HALF2: smaller images take FP32 decisions
+
+// Mean over the longest length inside the cloud shell of 16 x 4 rays of the image (0 for a ray below the
+// horizon); 1 if none rises.
+inline double crowding(const MarchLaunch& p) {
+    const float* v = p.u.camera.view;
+    const double tan = p.u.camera.camera_params[1], aspect = p.u.camera.camera_params[0];
+    const double h = (double)p.u.camera.camera_position[1] + 995000.0, outer = 1.018e6, inner = 1.0e6;
+    double sum = 0.0, most = 0.0;
+    for (int k = 0; k < 64; ++k) {
+        const double y = (2.0 * (k / 4 + 0.5) / 16.0 * p.height / p.uv_h - 1.0) * tan;
+        const double x = (2.0 * (k % 4 + 0.5) / 4.0 * p.width / p.uv_w - 1.0) * tan * aspect;
+        double d[3];
+        for (int i = 0; i < 3; ++i) d[i] = x * v[4 * i] - y * v[4 * i + 1] - v[4 * i + 2];
+        if (!(d[1] >= 0.0)) continue;
+        const double along2 = h * h * d[1] * d[1] / (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        const double off2 = h * h - along2;  // the ray's line passes the planet's centre at this distance squared
+        const double exit = sqrt(fmax(outer * outer - off2, 0.0)), enter = sqrt(fmax(inner * inner - off2, along2));
+        sum += fmax(exit - enter, 0.0);
+        most = fmax(most, exit - enter);
+    }
+    return most > 0.0 ? sum / 64.0 / most : 1.0;
+}
 
 // A team of kT lanes; the rays of a warp (32 / kT) as a pixel tile, the four warps of a block side by
 // side in a 2x2 arrangement.
@@ -1656,16 +1683,17 @@ int launch_tiled(const MarchLaunch& p0, cudaStream_t s, bool half2 = false, long
     // Kernels that the build knobs leave unused are not instantiated (if constexpr).
     const bool C = p.counters != nullptr;
     const dim3 block(MM_TILED_WARPS * 32);
-    const long long rays = (long long)gw * gh + beside;
+    const long long rays = (long long)gw * gh;
+    const double work = (double)(rays + beside) * (beside ? kCrowdingBeside : crowding(p));
     const bool h2 = !E && S == MM_SAMPLER_HARDWARE && half2 && p.pixel_mode != MM_PIXELS_PHASE16;
-    if (rays <= (h2 ? kHalf2Rays : kTeam2Rays)) {
-        if (rays <= kTeam8Rays)
+    if (work <= kTeam2Work && !(h2 && rays > kHalf2Rays)) {
+        if (work <= kTeam8Work)
             launch_team<E, S, 8, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
-        else if (rays <= kTeam4Rays)
+        else if (work <= kTeam4Work)
             launch_team<E, S, 4, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
         else
             launch_team<E, S, 2, 1, E ? 4 : 9>(p, gw, gh, s);
-    } else if (h2) {
+    } else if (h2 && rays > kHalf2Rays) {
         if constexpr (!E && S == MM_SAMPLER_HARDWARE) {
             if (C)
                 march_tiled_h2_kernel<true><<<grid, block, 0, s>>>(p);

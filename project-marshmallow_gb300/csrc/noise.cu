@@ -180,7 +180,7 @@ __device__ float value2(float qx, float qy, int f, uint32_t s) {
 // a product, a sum and a minimum each.  Every float operation is worley3's own, so the texels are the same
 // bytes.  Where an octave has more cells in reach than the table holds (more than about half a cell per
 // texel), its texels are computed one by one as before.
-// Bound by FP32 issue: 27 distances x 12 octaves a texel.  us at the start -> with the tables -> with packed FP32
+// Bound by FP32 issue: 27 distances x 12 octaves a texel.  us hashing every cell -> with the tables -> with packed FP32
 // operations -> 8 texels at a time: low-res 128^3 1229 -> 226 -> 201 -> 183, 64^3 164 -> 56 -> 52; hi-res 32^3
 // 27 -> 11, 64^3 109 -> 27 -> 25 -> 23.
 // (Passing over rows of cells no closer than the distance found so far costs what it saves: 232 -> 240.)
