@@ -28,6 +28,7 @@
 
 #include "mm_internal.h"
 #include "mm_math.h"
+#include "post_taps.h"
 
 namespace mm {
 
@@ -95,20 +96,14 @@ struct SoftTaps {
 // 1920x1080 111 -> 97, at 32 registers (all warps; 340 / 97 at 40, 639 / 163 with the compiler's choice).
 // Copying the alpha into a plane first, so that a tap touches a quarter of the bytes, costs more than it
 // saves: 372 / 107.
-struct InsideTaps {
+struct InsideTaps : TapArea {
     static constexpr unsigned kStride = 4;
     const float* p;
     unsigned row;
-    float w, h;
     unsigned origin;
     __device__ __forceinline__ InsideTaps(const PostLaunch& l)
-        : p(l.src + 3), row((unsigned)l.src_row), w((float)l.width), h((float)l.height),
+        : TapArea{(float)l.width, (float)l.height}, p(l.src + 3), row((unsigned)l.src_row),
           origin(0x4B400000u * (unsigned)l.src_row + 0x4B400000u * kStride) {}
-    // Whether a tap at (u, v) has its four texels inside; taps between two such taps of a line have them too.
-    __device__ __forceinline__ bool holds(float u, float v) const {
-        const float x = u * w - 0.5f, y = v * h - 0.5f;
-        return x >= 0.0f && x < w - 1.0f && y >= 0.0f && y < h - 1.0f;
-    }
     __device__ __forceinline__ float operator()(float u, float v) const {
         constexpr float kMagic = 12582912.0f;
         const float x = u * w - 0.5f, y = v * h - 0.5f;
@@ -125,13 +120,6 @@ struct TexTaps {
     cudaTextureObject_t t;
     __device__ __forceinline__ float operator()(float u, float v) const { return tex2D<float>(t, u, v); }
 };
-
-__device__ __forceinline__ void frag(int x, int y, int w, int h, float* px, float* py, float* u, float* v) {
-    *u = ((float)x + 0.5f) / (float)w;
-    *v = ((float)y + 0.5f) / (float)h;
-    *px = *u * 2.0f - 1.0f;
-    *py = *v * 2.0f - 1.0f;
-}
 
 // god-ray.frag:56-75 for the fragment at NDC (px, py) with centre alpha ca.
 template <class Taps>
@@ -150,23 +138,6 @@ __device__ __forceinline__ float god_ray_term(const PostLaunch& p, const Taps& a
         decay = decay * 0.99f;
     }
     return accum * 0.9f;
-}
-
-// radialBlur.frag:51-60: the mean of ten taps of the god-ray term along the line to the sun.
-template <class Taps>
-__device__ __forceinline__ float radial_term(const PostLaunch& p, const Taps& g, float px, float py) {
-    float lx = p.sun_x - px, ly = p.sun_y - py;
-    const float dist = sqrtf(lx * lx + ly * ly);
-    lx = lx / dist;
-    ly = ly / dist;
-    const float taps[10] = {-0.08f, -0.05f, -0.03f, -0.02f, -0.01f, 0.01f, 0.02f, 0.03f, 0.05f, 0.08f};
-    float accum = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 10; ++i) {
-        const float ox = taps[i] * lx * 1.5f * dist, oy = taps[i] * ly * 1.5f * dist;
-        accum = accum + g((px + ox) * 0.5f + 0.5f, (py + oy) * 0.5f + 0.5f) * 1.1f;
-    }
-    return accum / 10.0f;
 }
 
 __device__ __forceinline__ float uc2(float x) {  // tonemap.frag:11-14
@@ -252,16 +223,12 @@ __global__ void __launch_bounds__(256, kInside ? 8 : 1) radial_blur_kernel(PostL
         bool inside = false;
         if constexpr (kInside) {
             const InsideTaps taps(p);
-            // the outermost taps lie 0.12 of the way to the sun on either side; a little further out here,
-            // so that no rounding puts one of them beyond what is tested
-            const float ox = (p.sun_x - px) * 0.1201f, oy = (p.sun_y - py) * 0.1201f;
-            inside = taps.holds((px - ox) * 0.5f + 0.5f, (py - oy) * 0.5f + 0.5f) &&
-                     taps.holds((px + ox) * 0.5f + 0.5f, (py + oy) * 0.5f + 0.5f);
-            if (inside) a = radial_term(p, taps, px, py);
+            inside = radial_inside(taps, p.sun_x, p.sun_y, px, py);
+            if (inside) a = radial_term(p.sun_x, p.sun_y, taps, px, py);
         }
         if (!inside) {
             const SoftTaps alpha{Plane{p.src, p.src_pitch, 4, 3, p.width, p.height}};
-            a = radial_term(p, alpha, px, py);
+            a = radial_term(p.sun_x, p.sun_y, alpha, px, py);
         }
         o.x = p.kr * a + 0.5f * c.x;
         o.y = p.kg * a + 0.5f * c.y;
@@ -306,10 +273,10 @@ __global__ void __launch_bounds__(256) chain_kernel(PostLaunch p) {
         } else {
             float a;
             if (kTex) {
-                a = radial_term(p, TexTaps{p.gtex}, px, py);
+                a = radial_term(p.sun_x, p.sun_y, TexTaps{p.gtex}, px, py);
             } else {
                 const SoftTaps term{Plane{p.plane, p.plane_pitch, 1, 0, p.width, p.height}};
-                a = radial_term(p, term, px, py);
+                a = radial_term(p.sun_x, p.sun_y, term, px, py);
             }
             r = p.kr * a + 0.5f * c.x;
             g = p.kg * a + 0.5f * c.y;

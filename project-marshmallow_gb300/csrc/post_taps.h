@@ -1,0 +1,73 @@
+/*
+ * post_taps.h - the single post passes' radial-blur taps and the test that lets production arithmetic take them
+ * without clamps, for the kernels (post_kernel.cuh) and, compiled by a host compiler, for the tests.
+ */
+#ifndef MM_POST_TAPS_H_
+#define MM_POST_TAPS_H_
+
+#if defined(__CUDACC__)
+#define MM_TAPS_HD __host__ __device__ __forceinline__
+#else
+#define MM_TAPS_HD inline
+#endif
+
+#if !defined(__CUDA_ARCH__)
+#include <math.h>
+#endif
+
+namespace mm {
+namespace post {
+
+MM_TAPS_HD void frag(int x, int y, int w, int h, float* px, float* py, float* u, float* v) {
+    *u = ((float)x + 0.5f) / (float)w;
+    *v = ((float)y + 0.5f) / (float)h;
+    *px = *u * 2.0f - 1.0f;
+    *py = *v * 2.0f - 1.0f;
+}
+
+// radialBlur.frag:51-60: the mean of ten taps of the god-ray term along the line to the sun.
+template <class Taps>
+MM_TAPS_HD float radial_term(float sun_x, float sun_y, const Taps& g, float px, float py) {
+    float lx = sun_x - px, ly = sun_y - py;
+    const float dist = sqrtf(lx * lx + ly * ly);
+    lx = lx / dist;
+    ly = ly / dist;
+    const float taps[10] = {-0.08f, -0.05f, -0.03f, -0.02f, -0.01f, 0.01f, 0.02f, 0.03f, 0.05f, 0.08f};
+    float accum = 0.0f;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int i = 0; i < 10; ++i) {
+        const float ox = taps[i] * lx * 1.5f * dist, oy = taps[i] * ly * 1.5f * dist;
+        accum = accum + g((px + ox) * 0.5f + 0.5f, (py + oy) * 0.5f + 0.5f) * 1.1f;
+    }
+    return accum / 10.0f;
+}
+
+// The part of a w x h image where a bilinear tap has its four texels inside.
+struct TapArea {
+    float w, h;
+    // Whether a tap at (u, v) has its four texels inside; taps between two such taps of a line have them too.
+    // False for NaN.
+    MM_TAPS_HD bool holds(float u, float v) const {
+        const float x = u * w - 0.5f, y = v * h - 0.5f;
+        return x >= 0.0f && x < w - 1.0f && y >= 0.0f && y < h - 1.0f;
+    }
+};
+
+// Whether all taps of radial_term at (px, py) have their four texels inside.  On the sun radial_term divides 0
+// by 0 (as the shader does), and next to it a square could be flushed to zero: its taps are then NaN, which only
+// the clamped ones take.  The outermost taps lie 0.12 of the way to the sun on either side; a little further
+// out here, so that no rounding puts one of them beyond what is tested.
+MM_TAPS_HD bool radial_inside(const TapArea& a, float sun_x, float sun_y, float px, float py) {
+    const float lx = sun_x - px, ly = sun_y - py;
+    if (!(fabsf(lx) + fabsf(ly) > 1.0e-12f)) return false;
+    const float ox = lx * 0.1201f, oy = ly * 0.1201f;
+    return a.holds((px - ox) * 0.5f + 0.5f, (py - oy) * 0.5f + 0.5f) &&
+           a.holds((px + ox) * 0.5f + 0.5f, (py + oy) * 0.5f + 0.5f);
+}
+
+}  // namespace post
+}  // namespace mm
+
+#endif  // MM_POST_TAPS_H_

@@ -28,7 +28,8 @@ EXACT_UNITS = {"march_exact.cu", "march_exact_sw.cu", "noise.cu", "reproject.cu"
 FAST_UNITS = {"march_fast.cu", "surrogate.cu", "batch.cu", "reproject_fast.cu", "shadow.cu", "post.cu"}
 CUDA_UNITS = ["api.cu", "march_fast.cu", "march_exact.cu", "march_exact_sw.cu", "noise.cu", "peaks.cu", "noalloc.cu", "mlp.cu", "surrogate.cu", "batch.cu", "reproject.cu", "reproject_fast.cu", "shadow.cu", "shadow_exact.cu", "post.cu", "post_exact.cu"]
 CXX_UNITS = ["scene.cpp", "assets.cpp"]
-HEADERS = ["mm_internal.h", "mm_math.h", "march_kernel.cuh", "tc.cuh", "shadow_kernel.cuh", "post_kernel.cuh"]
+HEADERS = ["mm_internal.h", "mm_math.h", "march_kernel.cuh", "tc.cuh", "shadow_kernel.cuh", "post_kernel.cuh",
+           "post_taps.h"]
 
 
 def nvcc():
