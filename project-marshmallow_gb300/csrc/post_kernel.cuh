@@ -121,25 +121,6 @@ struct TexTaps {
     __device__ __forceinline__ float operator()(float u, float v) const { return tex2D<float>(t, u, v); }
 };
 
-// god-ray.frag:56-75 for the fragment at NDC (px, py) with centre alpha ca.
-template <class Taps>
-__device__ __forceinline__ float god_ray_term(const PostLaunch& p, const Taps& alpha, float px, float py, float ca) {
-    const float weight_density = 1.0f / 8.0f * 0.75f;  // SAMPLE_WEIGHT * DENSITY
-    const float dx = (px - p.sun_x) * weight_density, dy = (py - p.sun_y) * weight_density;
-    float accum = ca * 0.5f;
-    float decay = 1.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        px = px - dx;
-        py = py - dy;
-        float amt = alpha(px * 0.5f + 0.5f, py * 0.5f + 0.5f) * 0.5f;
-        amt = amt * (1.0f / 8.0f * decay);
-        accum = accum + amt;
-        decay = decay * 0.99f;
-    }
-    return accum * 0.9f;
-}
-
 __device__ __forceinline__ float uc2(float x) {  // tonemap.frag:11-14
     return ((x * (0.15f * x + 0.1f * 0.5f) + 0.2f * 0.02f) / (x * (0.15f * x + 0.5f) + 0.2f * 0.3f)) - 0.02f / 0.3f;
 }
@@ -184,21 +165,12 @@ __global__ void __launch_bounds__(256, kInside ? 8 : 1) god_rays_kernel(PostLaun
         bool inside = false;
         if constexpr (kInside) {
             const InsideTaps taps(p);
-            // the line's ends: the fragment itself (one step before the first tap) and the eighth tap
-            const float step = 1.0f / 8.0f * 0.75f;
-            const float dx = (px - p.sun_x) * step, dy = (py - p.sun_y) * step;
-            float ex = px, ey = py;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                ex = ex - dx;
-                ey = ey - dy;
-            }
-            inside = taps.holds(px * 0.5f + 0.5f, py * 0.5f + 0.5f) && taps.holds(ex * 0.5f + 0.5f, ey * 0.5f + 0.5f);
-            if (inside) term = god_ray_term(p, taps, px, py, c.w);
+            inside = god_ray_inside(taps, p.sun_x, p.sun_y, px, py);
+            if (inside) term = god_ray_term(p.sun_x, p.sun_y, taps, px, py, c.w);
         }
         if (!inside) {
             const SoftTaps alpha{Plane{p.src, p.src_pitch, 4, 3, p.width, p.height}};
-            term = god_ray_term(p, alpha, px, py, c.w);
+            term = god_ray_term(p.sun_x, p.sun_y, alpha, px, py, c.w);
         }
     }
     if (p.plane) {
@@ -316,7 +288,7 @@ __global__ void __launch_bounds__(256) god_rays_tex_kernel(PostLaunch p) {
     frag(x, y, p.width, p.height, &px, &py, &u, &v);
     const float ca = *(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p.aplane) + (size_t)y * p.plane_pitch) + x);
     *(reinterpret_cast<float*>(reinterpret_cast<char*>(p.plane) + (size_t)y * p.plane_pitch) + x) =
-        god_ray_term(p, TexTaps{p.atex}, px, py, ca);
+        god_ray_term(p.sun_x, p.sun_y, TexTaps{p.atex}, px, py, ca);
 }
 
 // which: 0 god rays, 1 radial blur, 2 tonemap, 3 chain (god-ray plane, then the fused kernel),

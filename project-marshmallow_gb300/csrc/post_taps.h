@@ -1,6 +1,6 @@
 /*
- * post_taps.h - the single post passes' radial-blur taps and the test that lets production arithmetic take them
- * without clamps, for the kernels (post_kernel.cuh) and, compiled by a host compiler, for the tests.
+ * post_taps.h - the single post passes' taps and the tests that let production arithmetic take them without
+ * clamps, for the kernels (post_kernel.cuh) and, compiled by a host compiler, for the tests.
  */
 #ifndef MM_POST_TAPS_H_
 #define MM_POST_TAPS_H_
@@ -25,6 +25,27 @@ MM_TAPS_HD void frag(int x, int y, int w, int h, float* px, float* py, float* u,
     *py = *v * 2.0f - 1.0f;
 }
 
+// god-ray.frag:56-75 for the fragment at NDC (px, py) with centre alpha ca.
+template <class Taps>
+MM_TAPS_HD float god_ray_term(float sun_x, float sun_y, const Taps& alpha, float px, float py, float ca) {
+    const float weight_density = 1.0f / 8.0f * 0.75f;  // SAMPLE_WEIGHT * DENSITY
+    const float dx = (px - sun_x) * weight_density, dy = (py - sun_y) * weight_density;
+    float accum = ca * 0.5f;
+    float decay = 1.0f;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int i = 0; i < 8; ++i) {
+        px = px - dx;
+        py = py - dy;
+        float amt = alpha(px * 0.5f + 0.5f, py * 0.5f + 0.5f) * 0.5f;
+        amt = amt * (1.0f / 8.0f * decay);
+        accum = accum + amt;
+        decay = decay * 0.99f;
+    }
+    return accum * 0.9f;
+}
+
 // radialBlur.frag:51-60: the mean of ten taps of the god-ray term along the line to the sun.
 template <class Taps>
 MM_TAPS_HD float radial_term(float sun_x, float sun_y, const Taps& g, float px, float py) {
@@ -44,21 +65,34 @@ MM_TAPS_HD float radial_term(float sun_x, float sun_y, const Taps& g, float px, 
     return accum / 10.0f;
 }
 
-// The part of a w x h image where a bilinear tap has its four texels inside.
+// The part of a w x h image where a bilinear tap has its four texels inside.  The ends of a line are tested here
+// and the taps on it computed elsewhere, in more steps and contracted as the compiler likes: eight subtractions
+// of positions up to 1 and a step off by 2^-23 of its size put a tap up to 8 * 2^-23 from where the end says, half
+// of that in (u, v), and two roundings more make the texel position: less than 6 * 2^-23 of the image's side.
+// The margin is 8 * 2^-23 of it.
+constexpr float kTapMargin = 1.0f / 1048576.0f;
 struct TapArea {
     float w, h;
-    // Whether a tap at (u, v) has its four texels inside; taps between two such taps of a line have them too.
-    // False for NaN.
+    // Whether a tap at (u, v) has its four texels inside by the margin; taps between two such taps of a line have
+    // them inside too.  False for NaN.
     MM_TAPS_HD bool holds(float u, float v) const {
-        const float x = u * w - 0.5f, y = v * h - 0.5f;
-        return x >= 0.0f && x < w - 1.0f && y >= 0.0f && y < h - 1.0f;
+        const float x = u * w - 0.5f, y = v * h - 0.5f, mx = kTapMargin * w, my = kTapMargin * h;
+        return x >= mx && x < w - 1.0f - mx && y >= my && y < h - 1.0f - my;
     }
 };
+
+// Whether all taps of god_ray_term at (px, py) have their four texels inside: the first and the eighth.
+MM_TAPS_HD bool god_ray_inside(const TapArea& a, float sun_x, float sun_y, float px, float py) {
+    const float step = 1.0f / 8.0f * 0.75f;
+    const float dx = (px - sun_x) * step, dy = (py - sun_y) * step;
+    return a.holds((px - dx) * 0.5f + 0.5f, (py - dy) * 0.5f + 0.5f) &&
+           a.holds((px - 8.0f * dx) * 0.5f + 0.5f, (py - 8.0f * dy) * 0.5f + 0.5f);
+}
 
 // Whether all taps of radial_term at (px, py) have their four texels inside.  On the sun radial_term divides 0
 // by 0 (as the shader does), and next to it a square could be flushed to zero: its taps are then NaN, which only
 // the clamped ones take.  The outermost taps lie 0.12 of the way to the sun on either side; a little further
-// out here, so that no rounding puts one of them beyond what is tested.
+// out here, since the division and the products after it round in proportion to the way.
 MM_TAPS_HD bool radial_inside(const TapArea& a, float sun_x, float sun_y, float px, float py) {
     const float lx = sun_x - px, ly = sun_y - py;
     if (!(fabsf(lx) + fabsf(ly) > 1.0e-12f)) return false;

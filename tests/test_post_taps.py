@@ -38,11 +38,13 @@ def _suns(w, h):
     return suns
 
 
-@pytest.mark.parametrize("w,h", [(1, 1), (2, 3), (3, 3), (33, 9), (257, 129), (641, 361), (640, 360), (1367, 7)])
-def test_radial_taps_are_inside(taps, w, h):
+@pytest.mark.parametrize("which", ["scan_radial", "scan_god_rays"])
+@pytest.mark.parametrize("w,h", [(1, 1), (2, 3), (3, 3), (33, 9), (257, 129), (641, 361), (640, 360), (1367, 7),
+                                 (32768, 5)])
+def test_taps_are_inside(taps, which, w, h):
     most = 0
     for sx, sy in _suns(w, h):
-        inside, bad = _scan(taps.scan_radial, w, h, sx, sy)
+        inside, bad = _scan(getattr(taps, which), w, h, sx, sy)
         assert bad == 0, (sx, sy, inside, bad)
         most = max(most, inside)
     if min(w, h) > 100:
