@@ -1038,6 +1038,12 @@ struct ConePool {
 // 12 blocks of the pooled kernel, 1 KB reserved for each, fill a 64 KB carveout.
 static_assert(MM_TILED_WARPS != 4 || sizeof(ConePool) <= 4352, "pool size");
 
+// An empty pool for the calling warp, whose lanes all call it: lanes append only behind the barrier.
+__device__ __forceinline__ void pool_reset(ConePool& q) {
+    if ((threadIdx.x & 31) == 0) q.waiting[threadIdx.x >> 5] = 0;
+    __syncwarp();
+}
+
 // One round: the `take` (<= 32) oldest records of the warp's pool, one per lane, then each owner's
 // blends in pool order.  Every lane of the warp calls it with the same head and take.
 // Cone taps a lane issues together: G.
@@ -1102,7 +1108,7 @@ __device__ __forceinline__ void march_pixel_q(const MarchLaunch& p, const Frame&
         // 2705 us, 1920x1080 789 -> 779 (10 blocks of 48: 2759 / 790; a 100 KB carveout 2712 / 781).
         store_pixel(p, px, py, make_float4(r.bg.x, r.bg.y, r.bg.z, r.alpha), CUDART_INF_F);
     }
-    if (lane == 0) q.waiting[wp] = 0;
+    pool_reset(q);
     float accum = 0.0f, trans = 1.0f;
     float stepSize = 0.05f * f.thickness;  // :390
     bool noHits = true;
@@ -1111,7 +1117,6 @@ __device__ __forceinline__ void march_pixel_q(const MarchLaunch& p, const Frame&
     float firstT = CUDART_INF_F;
     float t = r.t0;
     bool alive = live && t < r.t1;  // :408, the loop condition on entry
-    __syncwarp();
     // A trip is one iteration of every ray still marching, so its number is the rays' iteration count.
     // Issue bounds the loop (80% of the slots, 748 M warp instructions at 1920x1080), so a trip does no
     // more than it must: the opacity is looked at where it changes, and two votes tell whether anything
@@ -1347,7 +1352,7 @@ __device__ __forceinline__ void team_ray(const MarchLaunch& p, const Frame& f, c
                                          int px, int py, bool inside, int member, int base) {
     const unsigned full = 0xffffffffu;
     const int wp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) q.waiting[wp] = 0;
+    pool_reset(q);
     int head = 0, pending = 0;  // records of the warp's pool consumed / waiting (the same in every lane)
     Work w;
     Ray r{};
