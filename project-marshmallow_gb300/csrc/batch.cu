@@ -6,10 +6,11 @@
 // consecutive tiles from one global counter, find the view by a binary search over the views'
 // first-tile indices, read that view's record from constant memory and march the tile's rays
 // exactly as march_tiled_kernel does; within a view the tile rows just above its horizon come first.
-// The record upload, the counter reset and the kernel are captured into a CUDA graph once per (view
-// count, options, textures) and replayed for later batches.  MM_BATCH_BLOCKS is one ordinary launch over
-// 16x8-pixel blocks of all views instead: blocks of one SM then cover compact neighbouring tiles, as in
-// march_tiled_kernel.  The default schedule (MM_BATCH_GRAPH) launches the views' own kernels on up to 16
+// The record upload (views and textures), the counter reset and the kernel are captured into a CUDA graph
+// once per (view count, options) and replayed for later batches.  MM_BATCH_BLOCKS is one ordinary launch
+// over 16x8-pixel blocks of all views instead: blocks of one SM then cover compact neighbouring tiles, as in
+// march_tiled_kernel.  Its grid is part of its graph, so that is captured anew when the number of blocks
+// changes.  The default schedule (MM_BATCH_GRAPH) launches the views' own kernels on up to 16
 // concurrent branches.
 #include <cuda_runtime.h>
 #include <stdio.h>
@@ -144,6 +145,8 @@ struct BatchState {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;  // the last batch that read the staging buffers
     int g_n = -1, g_tw = 0, g_grab = 0, g_grid = 0, g_launches = 0, g_sched = -1;
+    // MM_BATCH_BLOCKS: the grids of the graph's launches
+    int g_blocks[(mm::batch::kMaxViews + mm::batch::kViewsPerLaunch - 1) / mm::batch::kViewsPerLaunch] = {};
     // MM_BATCH_GRAPH: one stream per branch and their fork/join events
     static constexpr int kBranches = 16;
     cudaStream_t branch[kBranches] = {};
@@ -247,6 +250,21 @@ int ensure_capacity(BatchState* b, int n) {
     return MM_OK;
 }
 
+// Blocks of the staged records' launch group that starts at view v0 (MM_BATCH_BLOCKS).
+int staged_blocks(const BatchState* b, int v0, int n) {
+    using mm::batch::kViewsPerLaunch;
+    const int m = n - v0 < kViewsPerLaunch ? n - v0 : kViewsPerLaunch;
+    return b->h_first[(size_t)(v0 / kViewsPerLaunch) * (kViewsPerLaunch + 1) + m];
+}
+
+// Whether the graph's launches have the grids that the staged records need.
+bool same_grids(const BatchState* b, int n, int sched) {
+    if (sched != MM_BATCH_BLOCKS) return true;
+    for (int v0 = 0; v0 < n; v0 += mm::batch::kViewsPerLaunch)
+        if (b->g_blocks[v0 / mm::batch::kViewsPerLaunch] != staged_blocks(b, v0, n)) return false;
+    return true;
+}
+
 // One launch per group of up to kViewsPerLaunch views: records to constant memory, counter reset,
 // persistent kernel.  Returns the number of launches through *launches.
 int enqueue(mm_context ctx, BatchState* b, int n, int tw, int grab, int grid, int sched, cudaStream_t s,
@@ -261,7 +279,7 @@ int enqueue(mm_context ctx, BatchState* b, int n, int tw, int grab, int grid, in
         MM_CUDA_TRY(cudaMemcpyToSymbolAsync(mm::batch::c_first_tile, first, (m + 1) * sizeof(int), 0,
                                             cudaMemcpyHostToDevice, s));
         if (sched == MM_BATCH_BLOCKS) {
-            mm::batch::batch_blocks_kernel<<<first[m], MM_TILED_WARPS * 32, 0, s>>>(m);
+            mm::batch::batch_blocks_kernel<<<staged_blocks(b, v0, n), MM_TILED_WARPS * 32, 0, s>>>(m);
         } else {
             MM_CUDA_TRY(cudaMemsetAsync(ctx->d_work + 2, 0, sizeof(unsigned int), s));
             mm::batch::Queue q;
@@ -400,7 +418,7 @@ extern "C" int mm_clouds_march_batch(mm_context ctx, const mm_view* views, int n
         return r;
     }
     if (!b->exec || b->g_n != n || b->g_tw != o.warp_tile_w || b->g_grab != o.tiles_per_grab || b->g_grid != grid ||
-        b->g_sched != o.schedule) {
+        b->g_sched != o.schedule || !same_grids(b, n, o.schedule)) {
         drop_graph(b);
         cudaStream_t cap_stream;
         MM_CUDA_TRY(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
@@ -431,6 +449,8 @@ extern "C" int mm_clouds_march_batch(mm_context ctx, const mm_view* views, int n
         b->g_grid = grid;
         b->g_sched = o.schedule;
         b->g_launches = launches;
+        if (o.schedule == MM_BATCH_BLOCKS)
+            for (int v0 = 0; v0 < n; v0 += K) b->g_blocks[v0 / K] = staged_blocks(b, v0, n);
     }
     // The graph copies the pinned staging buffers, which hold this batch's records now.
     MM_CUDA_TRY(cudaGraphLaunch(b->exec, s));
