@@ -154,7 +154,7 @@ __device__ __forceinline__ float4 ld4(const float* base, size_t pitch, int x, in
 // god-ray.frag as one pass: dst = (src.rgb, term) (plane == nullptr) or the term alone into the plane.
 // kInside: pixels whose taps all lie inside the image take InsideTaps (production).
 template <bool E, bool kInside>
-__global__ void __launch_bounds__(256, kInside ? 8 : 1) god_rays_kernel(PostLaunch p) {
+__global__ void __launch_bounds__(256, 8) god_rays_kernel(PostLaunch p) {
     const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
     if (x >= p.width || y >= p.height) return;
     const float4 c = ld4(p.src, p.src_pitch, x, y);
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256, kInside ? 8 : 1) god_rays_kernel(PostLaun
 
 // radialBlur.frag as one pass: dst = (k * blur(src.a) + 0.5 src.rgb, 1).  kInside as for god_rays_kernel.
 template <bool E, bool kInside>
-__global__ void __launch_bounds__(256, kInside ? 8 : 1) radial_blur_kernel(PostLaunch p) {
+__global__ void __launch_bounds__(256, 8) radial_blur_kernel(PostLaunch p) {
     const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
     if (x >= p.width || y >= p.height) return;
     const float4 c = ld4(p.src, p.src_pitch, x, y);
