@@ -1244,9 +1244,18 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_MARCH_MIN_BLOCKS) marc
                      (E || S != MM_SAMPLER_HARDWARE) ? 0 : MM_LARGE_PAIR>(p);
 }
 
+// Resident blocks per SM of the pooled kernel.  The 40 registers of 12 blocks suit production arithmetic; the exact
+// forms behind the texture unit and the counts spill there: 1920x1080, 12 against 10 blocks (48 registers),
+// exact 2876 / 2758 us, counting 984 / 963.  Exact arithmetic with the software sampler, whose fetches wait
+// longer, is better off with the warps: 44.2 / 46.1 ms.
+template <bool E, int S, bool C>
+constexpr int pool_min_blocks() {
+    return C || (E && S == MM_SAMPLER_HARDWARE) ? MM_MARCH_MIN_BLOCKS : MM_POOL_MIN_BLOCKS;
+}
+
 // Full frames with deferred, pooled sun cones (above).
 template <bool E, int S, bool C>
-__global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_POOL_MIN_BLOCKS) march_tiled_pool_kernel(MarchLaunch p) {
+__global__ void __launch_bounds__(MM_TILED_WARPS * 32, (pool_min_blocks<E, S, C>())) march_tiled_pool_kernel(MarchLaunch p) {
     march_tiled_q_body<E, S, C, (MM_SPEC_CURL != 0)>(p);
 }
 
@@ -1646,7 +1655,7 @@ void pool_carveout() {
     if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess &&
         cudaFuncGetAttributes(&a, march_tiled_pool_kernel<E, S, C>) == cudaSuccess && per_sm > 0) {
-        const long long need = (long long)MM_POOL_MIN_BLOCKS * ((long long)a.sharedSizeBytes + reserved);
+        const long long need = (long long)pool_min_blocks<E, S, C>() * ((long long)a.sharedSizeBytes + reserved);
         int pct = MM_POOL_CARVEOUT_PCT > 0 ? MM_POOL_CARVEOUT_PCT : (int)((100 * need + per_sm - 1) / per_sm);
         pct = pct < 1 ? 1 : (pct > 100 ? 100 : pct);
         cudaFuncSetAttribute(march_tiled_pool_kernel<E, S, C>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
