@@ -1313,6 +1313,27 @@ __global__ void __launch_bounds__(MM_TILED_WARPS * 32, MM_PAIR_MIN_BLOCKS) march
 #endif
 constexpr double kCrowdingBeside = 0.37;
 constexpr double kTeam8Work = MM_TEAM8_WORK, kTeam4Work = MM_TEAM4_WORK, kTeam2Work = MM_TEAM2_WORK;
+
+// The lines of a launch (work up to which its rays get teams of 8, 4, 2), by what a sample costs.  The more
+// it costs to issue, the sooner the lanes of a team cost more than the shorter chain saves: exact arithmetic, and
+// the software sampler above all.  Production arithmetic with the software sampler does best in teams of 8 up to
+// the pooled kernel's line.  us by teams of 8 / 4 / 2 / pooled, "view, size (work in thousands)":
+//   exact, texture unit      pitch 12, 400x225 (32)  305 / 276 / 328 / 517     level, 512x360 (55)      471 / 435 / 363 / 558
+//                            level, 640x480 (91)     740 / 681 / 543 / 580     pitch 12, 640x480 (107)  915 / 847 / 640 / 613
+//   exact, software, ms      down 20, 512x360 (30)   3.8 / 4.2 / 4.2 / 5.1     level, 512x360 (55)      7.5 / 8.3 / 7.4 / 7.9
+//                            down 20, 800x480 (64)   7.5 / 8.2 / 7.5 / 7.2     pitch 12, 960x540 (185) 23.8 / 26.8 / 24.4 / 13.1
+//   production, software, ms pitch 12, 640x360 (82)  4.2 / 4.8 / 4.3 / 4.6     pitch 12, 640x480 (107)  5.3 / 6.1 / 5.4 / 5.3
+//                            pitch 25, 640x480 (120) 6.5 / 7.5 / 6.7 / 5.7     pitch 12, 960x540 (185)  8.8 / 10.1 / 8.8 / 7.0
+//   production, counting     pitch 12, 960x540 (185) 764 / 514 / 364 / 416     pitch 25, 960x540 (207)  957 / 633 / 437 / 424
+struct TeamLines {
+    double eight, four, two;
+};
+template <bool E, int S>
+constexpr TeamLines team_lines(bool counting) {
+    if (S == MM_SAMPLER_SOFTWARE) return E ? TeamLines{30000, 40000, 55000} : TeamLines{110000, 110000, 110000};
+    if (E) return {30000, 50000, 100000};
+    return {kTeam8Work, kTeam4Work, counting && kTeam2Work > 200000.0 ? 200000.0 : kTeam2Work};
+}
 constexpr long long kHalf2Rays = 262144;  // MM_MATH_FAST_HALF2: smaller images take FP32 decisions
 
 // Mean over the longest length inside the cloud shell of 16 x 4 rays of the image (0 for a ray below the
@@ -1700,13 +1721,18 @@ int launch_tiled(const MarchLaunch& p0, cudaStream_t s, bool half2 = false, long
     const long long rays = (long long)gw * gh;
     const double work = (double)(rays + beside) * (beside ? kCrowdingBeside : crowding(p));
     const bool h2 = !E && S == MM_SAMPLER_HARDWARE && half2 && p.pixel_mode != MM_PIXELS_PHASE16;
-    if (work <= kTeam2Work && !(h2 && rays > kHalf2Rays)) {
-        if (work <= kTeam8Work)
-            launch_team<E, S, 8, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
-        else if (work <= kTeam4Work)
-            launch_team<E, S, 4, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
-        else
-            launch_team<E, S, 2, 1, E ? 4 : 9>(p, gw, gh, s);
+    const TeamLines lines = team_lines<E, S>(C);
+    if (work <= lines.two && !(h2 && rays > kHalf2Rays)) {
+        if constexpr (!E && S == MM_SAMPLER_SOFTWARE) {
+            launch_team<E, S, 8, 2, 8>(p, gw, gh, s);
+        } else {
+            if (work <= lines.eight)
+                launch_team<E, S, 8, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
+            else if (work <= lines.four)
+                launch_team<E, S, 4, E ? 1 : 2, E ? 4 : 8>(p, gw, gh, s);
+            else
+                launch_team<E, S, 2, 1, E ? 4 : 9>(p, gw, gh, s);
+        }
     } else if (h2 && rays > kHalf2Rays) {
         if constexpr (!E && S == MM_SAMPLER_HARDWARE) {
             if (C)
