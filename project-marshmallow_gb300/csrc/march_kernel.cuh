@@ -1103,6 +1103,16 @@ __device__ __forceinline__ void march_pixel_q(const MarchLaunch& p, const Frame&
     if (inside) {
         r = ray_setup<E, S>(p, f, px, py);
         live = !r.killed;
+    }
+    // No sample for any ray of the warp (below the horizon, or from above the clouds): nothing to wait in the
+    // image, which such a launch would write twice and read back (1920x1080 from 30 km up 28.8 -> 26.7 us).
+    if (!__any_sync(full, live && r.t0 < r.t1)) {
+        if (inside)
+            store_pixel(p, px, py, live ? composite<E>(p.u, f, r.rd, r.bg, r.alpha, 0.0f, 1.0f)
+                                        : make_float4(r.bg.x, r.bg.y, r.bg.z, r.alpha), CUDART_INF_F);
+        return;
+    }
+    if (inside) {
         // The background waits in the image: four registers less through the march, which with a pool of
         // 63 records (12 blocks in the 64 KB carveout) lets 12 blocks of 40 registers pay: 3840x2160 2759 ->
         // 2705 us, 1920x1080 789 -> 779 (10 blocks of 48: 2759 / 790; a 100 KB carveout 2712 / 781).
