@@ -151,6 +151,10 @@ __device__ __forceinline__ float4 ld4(const float* base, size_t pitch, int x, in
     return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const char*>(base) + (size_t)y * pitch) + x);
 }
 
+// Whether all of the warp's lanes that come here together have `inside`: a warp with both kinds of pixels takes the
+// clamped taps for all of them instead of one loop after the other.
+__device__ __forceinline__ bool warp_agrees(bool inside) { return __all_sync(__activemask(), inside); }
+
 // god-ray.frag as one pass: dst = (src.rgb, term) (plane == nullptr) or the term alone into the plane.
 // kInside: pixels whose taps all lie inside the image take InsideTaps (production).
 template <bool E, bool kInside>
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(256, 8) god_rays_kernel(PostLaunch p) {
         bool inside = false;
         if constexpr (kInside) {
             const InsideTaps taps(p);
-            inside = god_ray_inside(taps, p.sun_x, p.sun_y, px, py);
+            inside = warp_agrees(god_ray_inside(taps, p.sun_x, p.sun_y, px, py));
             if (inside) term = god_ray_term(p.sun_x, p.sun_y, taps, px, py, c.w);
         }
         if (!inside) {
@@ -195,7 +199,7 @@ __global__ void __launch_bounds__(256, 8) radial_blur_kernel(PostLaunch p) {
         bool inside = false;
         if constexpr (kInside) {
             const InsideTaps taps(p);
-            inside = radial_inside(taps, p.sun_x, p.sun_y, px, py);
+            inside = warp_agrees(radial_inside(taps, p.sun_x, p.sun_y, px, py));
             if (inside) a = radial_term(p.sun_x, p.sun_y, taps, px, py);
         }
         if (!inside) {
