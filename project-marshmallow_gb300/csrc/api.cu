@@ -282,6 +282,9 @@ int mm_noise_generate(const mm_noise_desc* desc, mm_texture* out, void* stream) 
     if (!out) return fail(MM_ERR_INVALID_ARGUMENT, "noise: null output handle");
     mm_texture t = nullptr;
     if ((r = make_texture(w, h, d, ch, &t))) return r;
+    // A march reads the bound of its hi-res volume only; one that erodes with a texture of another kind takes every
+    // fetch.  (Textures made from texels may be either, and all get theirs.)
+    if (desc->kind != MM_NOISE_HIRES_WORLEY) t->erosion_max = nullptr;
     cudaStream_t s = (cudaStream_t)stream;
     if ((r = mm_noise_fill(desc, t->texels, (size_t)w * h * d * ch, stream)) || (r = find_erosion_max(t, s)) ||
         (r = build_hw_copy(t, MM_FORMAT_UNORM8, s))) {
