@@ -277,9 +277,12 @@ typedef enum mm_math_mode {
 typedef enum mm_schedule {
     MM_SCHEDULE_TILED = 0,      /* one thread marches one pixel start to end (the shader's own loop
                                    nest), 8x4 pixel tiles per warp, block rows just above the horizon
-                                   first, the sun cones deferred and computed 32 at a time; launches of
-                                   <= 600000 rays, bound by their longest rays, give each ray a team of
-                                   2, 4 or 8 lanes instead */
+                                   first, the sun cones deferred and computed 32 at a time; launches
+                                   bound by their longest rays give each ray a team of 2, 4 or 8 lanes
+                                   instead: the launch's rays times the mean over the longest path inside
+                                   the cloud shell decide, and what a sample costs in the arithmetic and
+                                   sampler asked for (fast math on the texture unit, a 60 degree camera
+                                   pitched up by 12: up to about 600000 rays) */
     MM_SCHEDULE_PERSISTENT = 1  /* persistent warps; each iteration evaluates one cloudTest per lane
                                    (a march step or a sun-cone tap); finished lanes take the next ray
                                    of their warp's 8x4 pixel tile (ballot compaction).  Full SIMT
@@ -443,7 +446,8 @@ int mm_batch_options_default(mm_batch_options* o);
  * blocks of all views in one grid (MM_BATCH_BLOCKS; one launch per 72 views), a persistent kernel
  * whose warps take tiles of all views from one queue (MM_BATCH_PERSISTENT), or the views' own launches
  * on concurrent branches forked from `stream` and joined into it (MM_BATCH_GRAPH).  The first two
- * replay a CUDA graph (use_graph; re-captured when the view count or the options change), and their
+ * replay a CUDA graph (use_graph; re-captured when the view count, the options or, for
+ * MM_BATCH_BLOCKS, the number of blocks changes), and their
  * host-side records are staged in pinned memory owned by the context: such a call waits for the
  * previous one of the same context to finish reading them. */
 int mm_clouds_march_batch(mm_context ctx, const mm_view* views, int n, const mm_scene_textures* tex,

@@ -1131,7 +1131,7 @@ __device__ __forceinline__ void march_pixel_q(const MarchLaunch& p, const Frame&
     // Issue bounds the loop (80% of the slots, 748 M warp instructions at 1920x1080), so a trip does no
     // more than it must: the opacity is looked at where it changes, and two votes tell whether anything
     // was appended (one trip in twelve) and whether any ray goes on: 3840x2160 2775 -> 2759 us, 1920x1080 797
-    // -> 789, 16 bytes of spills instead of 64.  (Records written behind the vote, at the lane's rank in it,
+    // -> 789.  (Records written behind the vote, at the lane's rank in it,
     // instead of behind an atomic where they arise: 2759 -> 2820.)
     for (int trip = 0;; ++trip) {
         bool pushed = false;
