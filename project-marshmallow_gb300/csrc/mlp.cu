@@ -183,25 +183,32 @@ struct SmemWeights {
     float pad_[3];
 };
 
+// kBehind: the optimizer may still write the weights when this kernel starts (launch_behind), so they are read from
+// L2; otherwise the L1 shares them between an SM's CTAs (inference of 4,096 samples 14.3 -> 13.4 us).
+template <bool kBehind, class T>
+__device__ __forceinline__ T weight(const T* p) {
+    return kBehind ? __ldcg(p) : __ldg(p);
+}
+
+template <bool kBehind>
 __device__ void load_weights(SmemWeights& sw, const float* __restrict__ P, const __nv_bfloat16* __restrict__ WB) {
-    // 8 consecutive inputs of one output row are one 16-byte core-matrix row: one vector copy each.  From
-    // L2: the optimizer may write them after this kernel has started (launch_behind).
+    // 8 consecutive inputs of one output row are one 16-byte core-matrix row: one vector copy each.
     const uint4* wb = reinterpret_cast<const uint4*>(WB);
     for (int i = threadIdx.x; i < kHid * kIn / 8; i += blockDim.x)
         *reinterpret_cast<uint4*>(sw.w1 + tc::kmajor_offset(i / (kIn / 8), (i % (kIn / 8)) * 8, kIn)) =
-            __ldcg(wb + OFFB_W1 / 8 + i);
+            weight<kBehind>(wb + OFFB_W1 / 8 + i);
     for (int i = threadIdx.x; i < kHid * kHid / 8; i += blockDim.x) {
         const int o = i / (kHid / 8), k = (i % (kHid / 8)) * 8;
-        *reinterpret_cast<uint4*>(sw.w2 + tc::kmajor_offset(o, k, kHid)) = __ldcg(wb + OFFB_W2 / 8 + i);
-        *reinterpret_cast<uint4*>(sw.w3 + tc::kmajor_offset(o, k, kHid)) = __ldcg(wb + OFFB_W3 / 8 + i);
+        *reinterpret_cast<uint4*>(sw.w2 + tc::kmajor_offset(o, k, kHid)) = weight<kBehind>(wb + OFFB_W2 / 8 + i);
+        *reinterpret_cast<uint4*>(sw.w3 + tc::kmajor_offset(o, k, kHid)) = weight<kBehind>(wb + OFFB_W3 / 8 + i);
     }
     for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
-        sw.b1[i] = __ldcg(P + OFF_B1 + i);
-        sw.b2[i] = __ldcg(P + OFF_B2 + i);
-        sw.b3[i] = __ldcg(P + OFF_B3 + i);
-        sw.w4[i] = __ldcg(P + OFF_W4 + i);
+        sw.b1[i] = weight<kBehind>(P + OFF_B1 + i);
+        sw.b2[i] = weight<kBehind>(P + OFF_B2 + i);
+        sw.b3[i] = weight<kBehind>(P + OFF_B3 + i);
+        sw.w4[i] = weight<kBehind>(P + OFF_W4 + i);
     }
-    if (threadIdx.x == 0) sw.b4 = __ldcg(P + OFF_B4);
+    if (threadIdx.x == 0) sw.b4 = weight<kBehind>(P + OFF_B4);
 }
 
 // ------------------------------------------------------------------------------ inference
@@ -273,7 +280,7 @@ __global__ void __launch_bounds__(128, 5) infer_kernel(const __nv_bfloat16* __re
     InferSmem& S = *reinterpret_cast<InferSmem*>(smem_raw);
     if (n_dev) n = min(n, (int)*n_dev);  // sample count written by an earlier kernel
     const int tid = threadIdx.x, warp = tid >> 5;
-    load_weights(S.w, P, WB);
+    load_weights<false>(S.w, P, WB);
     if (tid == 0) tc::mbar_init(&S.bar, 1);
     if (warp == 0) tc::tmem_alloc(&S.tslot, 64);
     tc::fence_before_sync();
@@ -548,7 +555,7 @@ __global__ void __launch_bounds__(256, 2) train_kernel(const __nv_bfloat16* __re
     if (tid == 0) tc::mbar_init(&S.bar, 1);
     if (warp == 0) tc::tmem_alloc(&S.tslot, 256);
     grid_wait();  // the parameters of the step before
-    load_weights(S.w, P, WB);
+    load_weights<true>(S.w, P, WB);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
